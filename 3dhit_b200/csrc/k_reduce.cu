@@ -180,8 +180,11 @@ struct KahanAcc {  // compensated running sum
 
 constexpr int MS_WARPS = 4;  // warps per k_mode_sums block
 
-// A warp takes 32 consecutive kz modes of one (kx, ky) row at a time (the
-// chunks are dealt to the warps of the grid in a fixed order).  Along a row
+// A warp takes 32 consecutive kz modes of the up to four rows (+-kx, +-ky) at
+// a time (the chunks are dealt to the warps of the grid in a fixed order):
+// those rows share k2, the shell index and the weight, so their |u|^2 are
+// added in registers first (12 loads in flight per lane) and everything after
+// that -- weight, shell, scan, bins -- is done once for the four.  Along a row
 // |k| and hence the shell index never decrease with kz, so the lanes of one
 // shell form contiguous runs: a segmented shuffle scan in lane order gives
 // each run's sum in its last lane, which adds it (Kahan) to the warp's own
@@ -189,6 +192,9 @@ constexpr int MS_WARPS = 4;  // warps per k_mode_sums block
 // lanes touch one bin.  E, Omega and the band energy are per-lane Kahan sums.
 // At the end the warps' bins are added in warp order and the scalars by a
 // fixed shuffle tree, so the result does not depend on scheduling.
+// The scan's 35 shuffles and its float64 adds bound the kernel when they are
+// done per row (256^3 float32: 165 us per launch with all four rows apart, 71
+// together; 0.43 of HBM).
 template <typename T>
 __global__ void __launch_bounds__(MS_WARPS * 32) k_mode_sums(ModeSumArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -201,26 +207,41 @@ __global__ void __launch_bounds__(MS_WARPS * 32) k_mode_sums(ModeSumArgs<T> a) {
   __syncthreads();
   const Geom& g = a.g;
   const int nck = (g.Mz + 31) / 32;
-  const long long nchunks = (long long)g.Mx * g.My * nck;
+  // classes of rows with equal |kx| (|ky|): rows c and M - c, c = 0 .. M/2
+  const int ncx = g.Mx / 2 + 1, ncy = g.My / 2 + 1;
+  const long long nchunks = (long long)ncx * ncy * nck;
   double* wb = bs + warp * nb3;
   double* wc = bc + warp * nb3;
   KahanAcc sE, sO, sB;
   for (long long ch = (long long)blockIdx.x * MS_WARPS + warp; ch < nchunks; ch += (long long)gridDim.x * MS_WARPS) {
     const long long row = ch / nck;
     const int k = (int)(ch % nck) * 32 + lane;
-    const int j = (int)(row % g.My), i = (int)(row / g.My);
+    const int j = (int)(row % ncy), i = (int)(row / ncy);
     const bool on = k < g.Mz;
     const int fx = full_pos(i, g.hx, g.Mx, g.Nx), fy = full_pos(j, g.hy, g.My, g.Ny);
+    const int i2 = g.Mx - i, j2 = g.My - j;  // the partner rows, where they are others
+    const bool px = i > 0 && i2 != i, py = j > 0 && j2 != j;
     double e[3] = {0.0, 0.0, 0.0};
     int s = 0x7fffffff;  // lanes past the row: a key no real shell has
     if (on) {
-      const long long off = (long long)i * a.c_x + (long long)j * a.c_y + k;
+      const V2<T>* p0 = a.u + (long long)i * a.c_x + (long long)j * a.c_y + k;
+      const long long ox = (long long)(i2 - i) * a.c_x, oy = (long long)(j2 - j) * a.c_y;
+      V2<T> v[4][3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        v[0][c] = p0[c * a.c_c];
+        v[1][c] = py ? p0[c * a.c_c + oy] : czero<T>();
+        v[2][c] = px ? p0[c * a.c_c + ox] : czero<T>();
+        v[3][c] = px && py ? p0[c * a.c_c + ox + oy] : czero<T>();
+      }
       const T k2 = k2_of(a.k.kx[fx], a.k.ky[fy], a.k.kz[k]);
       const double w = herm_weight(g, k);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const V2<T> v = a.u[c * a.c_c + off];
-        e[c] = w * ((double)v.x * v.x + (double)v.y * v.y);
+        double q[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) q[r] = (double)v[r][c].x * v[r][c].x + (double)v[r][c].y * v[r][c].y;
+        e[c] = w * ((q[0] + q[1]) + (q[2] + q[3]));
       }
       const double t = (e[0] + e[1]) + e[2];
       sE.add(t);
