@@ -283,7 +283,7 @@ template <typename T>
 cudaError_t launch_grad9_vjp(const V2<T>* G, V2<T>* ub, const Geom& gm, KTab<T> kt, T inv_n3, cudaStream_t st);
 
 cudaError_t launch_tcgemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, float* C, int ldc, int M,
-                          int N, int K, int* err, cudaStream_t st, int splits = 1, float* work = nullptr);
+                          int N, int K, int* err, cudaStream_t st);
 
 // Learned-closure MLP (k_mlp.cu).  Weights bf16 row-major: forward W^T of
 // layers 1-4 ([64][16], [64][64], [64][64], [16][64]; W1 row 15 of the input
@@ -292,15 +292,14 @@ struct MlpArgs {
   const __nv_bfloat16 *w1t, *w2t, *w3t, *w4t, *w2, *w3, *w4;
   const float *b2, *b3, *b4;
   const float* x;    // feature f of point p at x[f * x_sf + p * x_sp]
-  const float* tau;  // [P][6] targets (NULL: inference only)
-  float* y;          // output c of point p at y[c * y_sf + p * y_sp] (may be NULL when training)
+  const float* tau;  // [P][6] targets (training)
+  float* y;          // output c of point p at y[c * y_sf + p * y_sp] (inference)
   long long P, x_sf, x_sp, y_sf, y_sp;
   float inv_count;   // 1 / (P * 6)
-  __nv_bfloat16 *aT0, *aT1, *aT2, *aT3;     // [16|65][P] activations (+ ones row)
-  __nv_bfloat16 *dzT1, *dzT2, *dzT3, *dzT4;  // [64|64|64|16][P]
-  double* loss;      // [grid] partial sums of (y - tau)^2
+  float* part;       // training: [grid][MLP_PART] weight-gradient partial sums
+  double* loss;      // training: [grid] partial sums of (y - tau)^2
   int* err;
-  // vector-Jacobian mode (training instantiation): with ybar set, dL/dy of
+  // vector-Jacobian mode (training kernel): with ybar set, dL/dy of
   // point p, component c is ybar[c * yb_sf + p * yb_sp] (instead of the MSE
   // gradient of tau); with xbar set (and w1, the backward layer-1 weight W1
   // [16][64], rows 0-8 used), dL/dx of feature f goes to xbar[f * x_sf + p * x_sp]
@@ -309,8 +308,19 @@ struct MlpArgs {
   float* xbar;
   const __nv_bfloat16* w1;
 };
-size_t mlp_smem_bytes();
 cudaError_t launch_mlp(const MlpArgs& a, int grid, cudaStream_t st);
+// floats of one CTA's partial: dW1 [16][64], dW2 and dW3 [65][64], dW4 [65][16]
+constexpr int MLP_PART = 16 * 64 + 2 * 65 * 64 + 65 * 16;
+cudaError_t launch_mlp_train(const MlpArgs& a, int grid, cudaStream_t st);
+struct MlpSumArgs {
+  const float* part;
+  const double* loss_part;
+  int nparts;
+  float *dW1, *dW2, *dW3, *dW4;
+  double* loss;  // nullable
+  double loss_scale;
+};
+cudaError_t launch_mlp_sums(const MlpSumArgs& a, cudaStream_t st);
 
 struct SumArgs {
   const double* partial;

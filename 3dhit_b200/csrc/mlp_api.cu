@@ -1,8 +1,8 @@
 // C ABI of the learned-closure MLP (include/hit3d.h): inference and the
-// loss gradients of one training batch.  Training runs the fused k_mlp pass
-// (forward, loss gradient, backward through the layers) and then the four
-// weight-gradient GEMMs dW_l = a_{l-1}^T dz_l over the batch on the tensor
-// cores, split along the points.
+// loss gradients of one training batch.  Training runs one pass over the batch
+// (k_mlp_train: forward, loss gradient, backward through the layers and the
+// weight gradients, all on the tensor cores) and the sum of its CTAs' partials.
+#include <algorithm>
 #include <string>
 
 #include "hit3d.h"
@@ -15,17 +15,7 @@ int record_error(int code, const std::string& msg);
 namespace {
 using hit::MlpArgs;
 
-constexpr int MLP_GRID = 2 * 148;  // two 75 KB CTAs (256 TMEM columns each) per SM
-constexpr int GRAD_SPLITS = 296;
-constexpr long long ROWS = 16 + 3 * 65 + 3 * 64 + 16;  // feature-major rows of the workspace
-
-__global__ void k_loss(const double* part, int n, double scale, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s * scale;
-  }
-}
+constexpr int MLP_GRID = 2 * 148;  // two 97 KB CTAs (256 TMEM columns each) per SM
 
 int cuda_err(cudaError_t e, const char* what) {
   return hit::record_error(HIT_E_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
@@ -53,9 +43,10 @@ MlpArgs args_of(const hit_mlp_weights* w) {
 
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// One fused k_mlp pass over P points (forward, output cotangent, backward
-// through the layers; a.tau or a.ybar set) and the four weight-gradient GEMMs
-// dW_l = a_{l-1}^T dz_l; loss (nullable) receives the MSE loss.
+// One k_mlp_train pass over P points (forward, output cotangent, backward
+// through the layers and the weight gradients dW_l = a_{l-1}^T dz_l; a.tau or
+// a.ybar set) and the sum of its CTAs' partials; loss (nullable) receives the
+// MSE loss.
 int run_grads(MlpArgs a, int64_t P, void* ws, float* dW1, float* dW2, float* dW3, float* dW4, double* loss, int* err,
               cudaStream_t st, const char* who) {
   if (P < 16 || P % 16) return hit::record_error(HIT_E_INVALID, std::string(who) + ": P must be a positive multiple of 16");
@@ -63,41 +54,13 @@ int run_grads(MlpArgs a, int64_t P, void* ws, float* dW1, float* dW2, float* dW3
   a.P = P;
   a.inv_count = (float)(1.0 / ((double)P * 6.0));
   a.err = err;
-  __nv_bfloat16* b = static_cast<__nv_bfloat16*>(ws);
-  auto take = [&](int rows) {
-    __nv_bfloat16* r = b;
-    b += (size_t)rows * P;
-    return r;
-  };
-  a.aT0 = take(16);
-  a.aT1 = take(65);
-  a.aT2 = take(65);
-  a.aT3 = take(65);
-  a.dzT1 = take(64);
-  a.dzT2 = take(64);
-  a.dzT3 = take(64);
-  a.dzT4 = take(16);
-  unsigned char* rest = static_cast<unsigned char*>(ws) + align256((size_t)ROWS * P * 2);
-  float* work = reinterpret_cast<float*>(rest);
-  double* part = reinterpret_cast<double*>(rest + align256((size_t)GRAD_SPLITS * 65 * 64 * 4));
-  a.loss = part;
+  a.part = static_cast<float*>(ws);
+  a.loss = reinterpret_cast<double*>(static_cast<unsigned char*>(ws) + align256((size_t)MLP_GRID * hit::MLP_PART * 4));
   const int grid = (int)std::min<int64_t>((P + 127) / 128, MLP_GRID);
-  cudaError_t e = hit::launch_mlp(a, grid, st);
+  cudaError_t e = hit::launch_mlp_train(a, grid, st);
   if (e != cudaSuccess) return cuda_err(e, who);
-  const int K = (int)P, splits = (int)std::min<int64_t>(GRAD_SPLITS, P / 16);
-  struct G {
-    const __nv_bfloat16 *A, *B;
-    float* C;
-    int M, N;
-  } gs[4] = {{a.aT3, a.dzT4, dW4, 65, 16}, {a.aT2, a.dzT3, dW3, 65, 64}, {a.aT1, a.dzT2, dW2, 65, 64},
-             {a.aT0, a.dzT1, dW1, 16, 64}};
-  for (const G& g : gs) {
-    e = hit::launch_tcgemm(g.A, K, g.B, K, g.C, g.N, g.M, g.N, K, err, st, splits, work);
-    if (e != cudaSuccess) return cuda_err(e, who);
-  }
-  if (!loss) return HIT_OK;
-  k_loss<<<1, 32, 0, st>>>(part, grid, 1.0 / ((double)P * 6.0), loss);
-  e = cudaGetLastError();
+  const hit::MlpSumArgs s{a.part, a.loss, grid, dW1, dW2, dW3, dW4, loss, 1.0 / ((double)P * 6.0)};
+  e = hit::launch_mlp_sums(s, st);
   return e == cudaSuccess ? HIT_OK : cuda_err(e, who);
 }
 }  // namespace
@@ -129,8 +92,7 @@ int hit_mlp_forward(const hit_mlp_weights* w, const float* x, int64_t P, float* 
 
 int64_t hit_mlp_workspace_bytes(int64_t P) {
   if (P < 1) return 0;
-  return (int64_t)(align256((size_t)ROWS * P * 2) + align256((size_t)GRAD_SPLITS * 65 * 64 * 4) +
-                   align256(MLP_GRID * sizeof(double)));
+  return (int64_t)(align256((size_t)MLP_GRID * hit::MLP_PART * 4) + align256(MLP_GRID * sizeof(double)));
 }
 
 int hit_mlp_train_grads(const hit_mlp_weights* w, const float* x, const float* tau, int64_t P, void* ws, float* dW1,
@@ -154,7 +116,6 @@ int hit_mlp_vjp(const hit_mlp_weights* w, const void* w1, const float* x, int64_
   a.x = x;
   a.x_sf = x_sf;
   a.x_sp = x_sp;
-  a.tau = ybar;  // selects the training instantiation; the cotangent replaces the loss gradient
   a.ybar = ybar;
   a.yb_sf = y_sf;
   a.yb_sp = y_sp;

@@ -38,6 +38,12 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// The same with both operands MN-major ([k][m] tiles; transposed products).
+// An MN-major no-swizzle operand is the K-major tile above read the other way
+// round: 8 x 8 core matrices of 8 k rows of 16 bytes, descriptor SBO = the
+// stride between groups of 8 along M (or N), LBO = between groups of 8 along K.
+__host__ __device__ constexpr uint32_t idesc_bf16_tt(int M, int N) { return idesc_bf16(M, N) | (1u << 15) | (1u << 16); }
+
 // D(tmem) (+)= A(smem desc) * B(smem desc); issued by one thread.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
   asm volatile(

@@ -286,7 +286,7 @@ int64_t hit_mlp_workspace_bytes(int64_t P);
  * (P a multiple of 16): dW1 [16][64] (row 15 = d b1), dW2 and dW3 [65][64]
  * and dW4 [65][16] (row 64 = d b), float32 DEVICE arrays in [in][out]
  * order; loss_dev (DEVICE double) receives the loss.  The weight gradients
- * are tensor-core GEMMs over the points (split K). */
+ * are accumulated on the tensor cores, tile by tile, in the same pass. */
 int hit_mlp_train_grads(const hit_mlp_weights *w, const float *x,
                         const float *tau, int64_t P, void *workspace,
                         float *dW1, float *dW2, float *dW3, float *dW4,
