@@ -21,6 +21,7 @@
 
 #include "fft_core.cuh"
 #include "kernels.h"
+#include "p3_epilogue.cuh"
 #include "tc_common.cuh"
 #include "tma.cuh"
 
@@ -327,168 +328,6 @@ template <int N, int W, int NTH> __host__ __device__ constexpr bool p3_in_regs()
 // divergence k_j tau_hat_ij of the SGS stress.
 template <typename T, int N, int W, int NTH> __host__ __device__ constexpr bool p3_les() {
   return std::is_same<T, float>::value && !p3_in_regs<N, W, NTH>() && N <= 256;
-}
-
-// State rows of one mode for the epilogue: us = stage input (u for stages
-// 0/1), ac/uu = accumulator and u (stages 2..4).
-template <typename T>
-__device__ __forceinline__ void p3_load(const P3Args<T>& a, long long o, V2<T> (&us)[3], V2<T> (&ac)[3],
-                                        V2<T> (&uu)[3]) {
-  const V2<T>* __restrict__ pus = a.stage <= 1 ? a.u : a.s;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    us[c] = pus[c * a.c_c + o];
-    if (a.stage >= 2) {
-      ac[c] = a.acc[c * a.c_c + o];
-      uu[c] = a.u[c * a.c_c + o];
-    }
-  }
-}
-
-// RHS epilogue of one stored mode (x position pos, z index z, state offset
-// o): du holds the x-forward nonlinear term (u x w)^ on entry.  Forcing is
-// added before dealias and projection (navierstokes.py:88-92), then the
-// viscous term (navierstokes.py:95) and the RK4 stage algebra
-// (integrators.py:32-38); ns receives the new stage input (or new state) and
-// the float64 partial sums are accumulated.
-template <typename T>
-__device__ __forceinline__ void p3_point(const P3Args<T>& a, int pos, int fy, int z, T ky, T kz, T cf, long long o,
-                                         V2<T> (&du)[3], const V2<T> (&us)[3], const V2<T> (&ac)[3],
-                                         const V2<T> (&uu)[3], V2<T> (&ns)[3], double& sE, double& sO,
-                                         double& sB) {
-  const Geom& g = a.g;
-  const T kx = __ldg(a.k.kx + pos);
-  const T k2 = k2_of(kx, ky, kz);
-  const T ik2 = inv_k2_of(k2);
-  if (a.fext) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) du[c] = cadd(du[c], a.fext[c * a.c_c + o]);
-  }
-  if (a.forcing == 1) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) du[c] = cadd(du[c], cscale(us[c], a.fA));
-  } else if (a.forcing == 2) {
-    if (a.kmin2 <= k2 && k2 <= a.kmax2) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) du[c] = cadd(du[c], cscale(us[c], cf));
-    }
-  } else if (a.forcing == 3) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) du[c] = cadd(du[c], cscale(us[c], cf));
-  }
-  // every stored mode of the dealiased path lies inside the 2/3 box
-  if (g.pruned ? (pos | fy | z) == 0 : !in_dealias(g, pos, fy, z)) {
-    du[0] = du[1] = du[2] = czero<T>();
-  }
-  // projection: div = (kx d0 + ky d1 + kz d2) / k^2 ; d -= k div
-  V2<T> div;
-  div.x = (kx * du[0].x + ky * du[1].x + kz * du[2].x) * ik2;
-  div.y = (kx * du[0].y + ky * du[1].y + kz * du[2].y) * ik2;
-  du[0] = csub(du[0], cscale(div, kx));
-  du[1] = csub(du[1], cscale(div, ky));
-  du[2] = csub(du[2], cscale(div, kz));
-  const T nk2 = a.nu * k2;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) du[c] = csub(du[c], cscale(us[c], nk2));
-
-  V2<T>* __restrict__ pu = a.u;
-  V2<T>* __restrict__ pacc = a.acc;
-  V2<T>* __restrict__ ps = a.s;
-  V2<T>* __restrict__ pout = a.out;
-  if (a.ifrk && a.stage > 0) {
-    // integrating-factor (Lawson) RK4 with E = e^{-nu k^2 dt/2} and N the RHS
-    // without its viscous term:
-    //   s2 = E (u + dt/2 k1),  s3 = E u + dt/2 k2,  s4 = E^2 u + dt E k3,
-    //   u' = E^2 u + dt/6 ((E (E k1 + 2 k2) + 2 E k3) + k4)
-    // (acc holds E k1, then E (E k1 + 2 k2), then + 2 E k3)
-    const T E = visc_factor(a.nuh, k2);
-    switch (a.stage) {
-      case 1:
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          pacc[c * a.c_c + o] = cscale(du[c], E);
-          ns[c] = cscale(cadd(us[c], cscale(du[c], a.a_next)), E);
-          ps[c * a.c_c + o] = ns[c];
-        }
-        break;
-      case 2:
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          V2<T> acn = ac[c];
-          acn.x = acn.x + T(2) * du[c].x;
-          acn.y = acn.y + T(2) * du[c].y;
-          pacc[c * a.c_c + o] = cscale(acn, E);
-          ns[c] = cadd(cscale(uu[c], E), cscale(du[c], a.a_next));
-          ps[c * a.c_c + o] = ns[c];
-        }
-        break;
-      case 3:
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const V2<T> ek = cscale(du[c], E);
-          V2<T> acn = ac[c];
-          acn.x = acn.x + T(2) * ek.x;
-          acn.y = acn.y + T(2) * ek.y;
-          pacc[c * a.c_c + o] = acn;
-          ns[c] = cadd(cscale(uu[c], E * E), cscale(ek, a.a_next));
-          ps[c * a.c_c + o] = ns[c];
-        }
-        break;
-      default:
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const V2<T> acn = cadd(ac[c], du[c]);
-          ns[c] = cadd(cscale(uu[c], E * E), cscale(acn, a.dt6));
-          pu[c * a.c_c + o] = ns[c];
-        }
-        break;
-    }
-  } else switch (a.stage) {
-    case 0:
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        pout[c * a.c_c + o] = du[c];
-        ns[c] = czero<T>();
-      }
-      break;
-    case 1:
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        pacc[c * a.c_c + o] = du[c];
-        ns[c] = cadd(us[c], cscale(du[c], a.a_next));
-        ps[c * a.c_c + o] = ns[c];
-      }
-      break;
-    case 2:
-    case 3:
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        V2<T> acn = ac[c];
-        acn.x = acn.x + T(2) * du[c].x;
-        acn.y = acn.y + T(2) * du[c].y;
-        pacc[c * a.c_c + o] = acn;
-        ns[c] = cadd(uu[c], cscale(du[c], a.a_next));
-        ps[c * a.c_c + o] = ns[c];
-      }
-      break;
-    default:
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const V2<T> acn = cadd(ac[c], du[c]);
-        ns[c] = cadd(uu[c], cscale(acn, a.dt6));
-        pu[c * a.c_c + o] = ns[c];
-      }
-      break;
-  }
-  if (a.partial) {
-    double a2 = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) a2 += (double)ns[c].x * ns[c].x + (double)ns[c].y * ns[c].y;
-    const double w = herm_weight(g, z);
-    sE += w * a2;
-    sO += w * (double)k2 * a2;
-    if (a.kmin2 <= k2 && k2 <= a.kmax2) sB += w * a2;
-  }
 }
 
 // Register mode: the epilogue runs in 8 passes, pass r over the positions
@@ -1229,6 +1068,7 @@ cudaError_t take_axis_timeout(int* flag) {
 
 template <typename T> int p3_tile_w(int Nx) {
   int w = 0;
+  if (xf_columns<T>(Nx)) return xf_tile_w<T>();
   dispatch_len(Nx, [&](auto nn) { w = tile_wp<T>(decltype(nn)::value); return cudaSuccess; });
   return w;
 }
@@ -1332,20 +1172,31 @@ template <int NN, int W> cudaError_t launch_p3m_v(const P3Args<float>& a, cudaSt
 // other work (on small grids, e.g. a closure on a second stream).
 template <int N> constexpr int p_threads() { return N <= 128 ? NTP / 2 : NTP; }
 
+// Columns with xf_columns take the field-parallel kernels of k_xfield.cu,
+// except the passes of the fused LES stage (12 x-inverse outputs, nine
+// x-forward fields; float32 only) and the standalone x-inverse of 256-point
+// columns on the general layout (k_p1 240 us, k_p1f 290 at 256^3), which k_p1 /
+// k_p3 run.
 template <typename T> cudaError_t launch_p1(const P1Args<T>& a, cudaStream_t st) {
+  if (xf_columns<T>(a.g.Nx) && !a.les && (a.g.Nx < 256 || a.g.pruned)) return launch_p1f<T>(a, st);
   return dispatch_len(a.g.Nx, [&](auto nn) {
     constexpr int NN = decltype(nn)::value;
-    return launch_p1_v<T, NN, tile_wp<T>(NN), p_threads<NN>()>(a, st);
+    if constexpr (!xf_columns<T>(NN) || std::is_same<T, float>::value)
+      return launch_p1_v<T, NN, tile_wp<T>(NN), p_threads<NN>()>(a, st);
+    else return cudaErrorInvalidValue;
   });
 }
 
 template <typename T> cudaError_t launch_p3(const P3Args<T>& a, cudaStream_t st) {
+  if (xf_columns<T>(a.g.Nx) && !a.les && a.fuse_p1 != 2) return launch_p3f<T>(a, st);
   return dispatch_len(a.g.Nx, [&](auto nn) {
     constexpr int NN = decltype(nn)::value;
     if constexpr (std::is_same<T, float>::value && NN == 512) {
       return launch_p3m_v<NN, tile_wp<float>(NN)>(a, st);
-    } else {
+    } else if constexpr (!xf_columns<T>(NN) || std::is_same<T, float>::value) {
       return launch_p3_v<T, NN, tile_wp<T>(NN), p_threads<NN>()>(a, st);
+    } else {
+      return cudaErrorInvalidValue;
     }
   });
 }

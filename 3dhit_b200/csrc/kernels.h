@@ -41,6 +41,14 @@ template <typename T> __host__ __device__ constexpr int tile_w(int N) {
 // k_p1/k_p3 tile width (same as the axis kernels).
 template <typename T> __host__ __device__ constexpr int tile_wp(int N) { return tile_w<T>(N); }
 
+// Column lengths of the field-parallel x kernels (k_xfield.cu) and their tile
+// width.  Longer columns do not fit five exchange tiles per CTA with two CTAs
+// on an SM; float64 columns of 256 points just do on the dealiased layout (433
+// us against k_p3's 428 per launch at 256^3) and not on the general one (1578
+// against 1100), so they stay with k_p3.
+template <typename T> __host__ __device__ constexpr bool xf_columns(int N) { return N <= (sizeof(T) == 4 ? 256 : 128); }
+template <typename T> __host__ __device__ constexpr int xf_tile_w() { return 64 / (int)sizeof(V2<T>); }
+
 // Plain column FFT along a strided axis ("a") of a 4-D array indexed
 // (comp, a, o, z): element at src + c*s_c + a*s_a + o*s_o + z.  Input rows
 // along a are compact (Min stored rows, hin non-negative), output rows compact
@@ -77,8 +85,10 @@ template <typename T> struct P3Args {
   const V2<T>* t3;  // (3, Nx, My, Mzp)
   long long t_c, t_x;
   V2<T>* u;         // state (3, Mx, My, Mzp)
+  V2<T>* u_out;     // new state (stage 4)
   V2<T>* acc;       // RK accumulator
   V2<T>* s;         // stage input of stages 2..4
+  V2<T>* s_out;     // new stage input (stages 1..3)
   V2<T>* out;       // stage 0: du output
   long long c_c, c_x;
   V2<T>* t6;        // fused P1 output
@@ -193,6 +203,9 @@ template <typename K> int resident_grid(K kernel, int threads, size_t smem, long
 template <typename T> cudaError_t launch_axis(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, int nc, cudaStream_t st);
 template <typename T> cudaError_t launch_p1(const P1Args<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_p3(const P3Args<T>& a, cudaStream_t st);
+// columns with xf_columns (k_xfield.cu)
+template <typename T> cudaError_t launch_p1f(const P1Args<T>& a, cudaStream_t st);
+template <typename T> cudaError_t launch_p3f(const P3Args<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_zcross(int H, const ZCrossArgs<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_zc2r(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st);
 template <typename T> cudaError_t launch_zr2c(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st);

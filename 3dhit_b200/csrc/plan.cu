@@ -428,9 +428,15 @@ int launch_p2_les(hit_plan* p, Path& P, const hit_mlp_weights& w, int* err, cuda
 // les_in: the fused LES stage (x-forward of T12's nine fields, the force
 // -i k_j tau_hat_ij added and stored in FEXT); les_next: the fused x-inverse
 // is the LES one (12 fields into T12), for a following fused LES stage.
+// u, s_in, s_out, u_out: the step's state, the stage's input, the next stage's
+// input and the step's result (P.U, P.S, P.S, P.U unless given).
+template <typename T> struct StageBufs {
+  V2<T>*u = nullptr, *s_in = nullptr, *s_out = nullptr, *u_out = nullptr;
+};
 template <typename T>
 int launch_p3_stage(hit_plan* p, Path& P, const Scalars& s, int stage, double dt, bool fuse, bool partial,
-                    const V2<T>* fext, cudaStream_t st, bool les_in = false, bool les_next = false) {
+                    const V2<T>* fext, cudaStream_t st, bool les_in = false, bool les_next = false,
+                    const StageBufs<T>& b = StageBufs<T>{}) {
   const Geom& g = P.g;
   P3Args<T> a{};
   a.t3 = vp<T>(les_in ? P.t12 : P.t6);
@@ -438,9 +444,11 @@ int launch_p3_stage(hit_plan* p, Path& P, const Scalars& s, int stage, double dt
   a.fext_out = les_in ? vp<T>(P.FEXT) : nullptr;
   a.t_c = (long long)g.Nx * g.My * g.Mzp;
   a.t_x = (long long)g.My * g.Mzp;
-  a.u = vp<T>(P.U);
+  a.u = b.u ? b.u : vp<T>(P.U);
+  a.u_out = b.u_out ? b.u_out : a.u;
   a.acc = vp<T>(P.ACC);
-  a.s = vp<T>(P.S);
+  a.s = b.s_in ? b.s_in : vp<T>(P.S);
+  a.s_out = b.s_out ? b.s_out : a.s;
   a.out = vp<T>(P.D);
   a.c_c = (long long)g.Mx * g.My * g.Mzp;
   a.c_x = (long long)g.My * g.Mzp;
