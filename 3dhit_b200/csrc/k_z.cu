@@ -23,69 +23,11 @@
 #include "kernels.h"
 #include "mlp_core.cuh"
 #include "tma.cuh"
+#include "zrow.cuh"
 #include "zwarp.cuh"
 
 namespace hit {
 
-template <int H> __host__ __device__ constexpr int z_rows_per_block() {
-  return (512 / H) > 32 ? 32 : (512 / H < 1 ? 1 : 512 / H);
-}
-// threads per block: one per last-stage butterfly of the 3*RB forward rows
-template <int H> __host__ __device__ constexpr int z_threads() {
-  return ((3 * z_rows_per_block<H>() * (H / fft16_radix(H, fft16_nstages(H) - 1)) + 31) / 32 * 32) < 96
-             ? 96
-             : ((3 * z_rows_per_block<H>() * (H / fft16_radix(H, fft16_nstages(H) - 1)) + 31) / 32 * 32);
-}
-// rows of Mzp entries are at most this long (Mzp <= round_up(H+1, 8))
-template <int H> __host__ __device__ constexpr int z_row_cap() { return (H + 1 + 7) / 8 * 8; }
-
-// conj-paired pre-processing of one c2r row element k in [0, H).
-template <typename T>
-__device__ __forceinline__ V2<T> c2r_pre(const V2<T>* row, int k, int H, int Mz, const V2<T>* twz) {
-  V2<T> X = k < Mz ? row[k] : czero<T>();
-  const int kk = H - k;  // in [1, H]
-  V2<T> Y = kk < Mz ? row[kk] : czero<T>();
-  if (k == 0) {
-    X.y = T(0);
-    Y.y = T(0);  // kk == H: Nyquist
-  }
-  Y.y = -Y.y;  // conj X[H-k]
-  const V2<T> s = cadd(X, Y), d = csub(X, Y);
-  V2<T> w = twz[k];
-  w.y = -w.y;  // e^{+2 pi i k / Nz}
-  return cadd(s, cmul_i(cmul(w, d)));
-}
-
-// r2c post-processing: output bin k in [0, H] from Z (length H), Z[i] = z(i).
-// HALVE = false returns twice the bin (for callers that fold the 1/2 into
-// their input scale).
-template <typename T, bool HALVE = true, class ZF>
-__device__ __forceinline__ V2<T> r2c_post(ZF&& z, int k, int H, const V2<T>* twz) {
-  const V2<T> a = z(k == H ? 0 : k);
-  V2<T> b = z(k == 0 ? 0 : H - k);
-  b.y = -b.y;
-  V2<T> E = cadd(a, b), O = cmul_mi(csub(a, b));
-  if constexpr (HALVE) {
-    E = cscale(E, T(0.5));
-    O = cscale(O, T(0.5));
-  }
-  const V2<T> w = twz[k];  // e^{-2 pi i k / Nz}
-  return cadd(E, cmul(w, O));
-}
-
-// Shared twiddles of the z kernels: the FFT stage tables (length H, radix-16
-// plan) followed by exp(-2 pi i k / Nz) for k in [0, H].
-template <int H> __host__ __device__ constexpr int z_tw_slots() { return (tw_size<true>(H) + H + 1 + 1) / 2 * 2; }
-// (an even slot count keeps whatever follows the tables 16-byte aligned)
-template <typename T, int H, int NTH>
-__device__ __forceinline__ void fill_z_twiddles(V2<T>* tws, const V2<T>* __restrict__ tw) {
-  fill_stage_twiddles<T, H, true, NTH>(tws, tw);
-  V2<T>* twz = tws + tw_size<true>(H);
-  for (int k = threadIdx.x; k <= H; k += NTH) twz[k] = tw[k * (TWN / (2 * H))];
-  __syncthreads();
-}
-
-constexpr int Z_WAIT = 1 << 22;  // mbarrier polls before a TMA wait gives up
 __device__ int g_z_timeout = 0;   // set when a TMA wait gave up (hit_device_status)
 // Polls of the wait for a row group (hit_set_wait_limit lowers it so that a
 // test can make the wait give up); the wait for the copies still in flight
@@ -364,11 +306,6 @@ __global__ void __launch_bounds__(128, 4) k_zles(ZLesArgs a) {
 // shuffle; outputs are written over the first three input fields of the row.
 
 constexpr int ZW_MINB = 3;  // CTAs per SM the register budget is sized for
-// DA: the dealiased layout, Mz = Nz/3 + 1 and Mzp = Mz rounded up to 8 as
-// compile-time constants, so the bounds of the pre-processing loads and of
-// the outputs fold into each value's position range (known-zero inputs are
-// not loaded, outputs past the row are not formed).
-template <int H> constexpr int zw_da_mz() { return (2 * H) / 3 + 1; }
 template <int H, int NWARP, bool DA>
 __global__ void __launch_bounds__(NWARP * 32, ZW_MINB) k_zwarp(ZCrossArgs<float> a) {
   using Z = ZW<H>;
@@ -817,21 +754,6 @@ cudaError_t take_z_timeout(int* flag) {
   return v ? cudaMemcpyToSymbol(g_z_timeout, &zero, sizeof(int)) : cudaSuccess;
 }
 
-template <typename F> cudaError_t dispatch_half(int H, F&& f) {
-  switch (H) {
-    case 2: return f(std::integral_constant<int, 2>{});
-    case 4: return f(std::integral_constant<int, 4>{});
-    case 8: return f(std::integral_constant<int, 8>{});
-    case 16: return f(std::integral_constant<int, 16>{});
-    case 32: return f(std::integral_constant<int, 32>{});
-    case 64: return f(std::integral_constant<int, 64>{});
-    case 128: return f(std::integral_constant<int, 128>{});
-    case 256: return f(std::integral_constant<int, 256>{});
-    case 512: return f(std::integral_constant<int, 512>{});
-    default: return cudaErrorInvalidValue;
-  }
-}
-
 template <typename T, int H> constexpr size_t zr2c_smem() {
   return sizeof(V2<T>) * (z_rows_per_block<H>() * skew_ld(H) + z_tw_slots<H>());
 }
@@ -929,7 +851,17 @@ template <typename T> cudaError_t launch_zcross(int H, const ZCrossArgs<T>& a, c
   }
   return dispatch_half(H, [&](auto hh) {
     constexpr int HH = decltype(hh)::value;
-    return launch_zcross_v<T, HH, z_rows_per_block<HH>(), z_threads<HH>(), 4>(a, st);
+    // Rows per CTA group.  float64 takes half the rows of float32: its groups
+    // fill 110 KB otherwise, two CTAs (six warps) per SM (z pass 82 -> 62 us at
+    // 128^3, 580 -> 408 at 256^3; a quarter: 83 and 678).  Grids with few rows
+    // take a sixteenth, so that every SM has groups (32 x 32 rows of 32 points
+    // in groups of 32 ran on 32 CTAs: 18.9 us; in groups of 2: 8.5; 64^3 float64
+    // step 153 -> 142 us).
+    constexpr int RB0 = z_rows_per_block<HH>();
+    constexpr int RB = sizeof(T) == 8 && RB0 > 1 ? RB0 / 2 : RB0;
+    constexpr int RS = RB0 / 16 < 1 ? 1 : RB0 / 16;
+    if (RS < RB && a.nrows < 4 * 148 * RB) return launch_zcross_v<T, HH, RS, z_threads<HH>(), 4>(a, st);
+    return launch_zcross_v<T, HH, RB, z_threads<HH>(), 4>(a, st);
   });
 }
 
