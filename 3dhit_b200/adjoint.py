@@ -27,7 +27,7 @@ from . import _native as nat
 from .forcing import BandForcing, LinearForcing, native_params
 from .grid import _check_state
 from .integrators import rollout
-from .navierstokes import NSParams, NSRHS
+from .navierstokes import NSParams, NSRHS, resolve_flags
 
 __all__ = ["rhs_vjp", "rk4_step_vjp", "rollout_vjp", "rollout_autograd", "PARAM_NAMES"]
 
@@ -43,6 +43,8 @@ def _setup(rhs, params, u_hat, ct):
     g = rhs.grid
     u_hat = _check_state(u_hat, g)
     ct = _check_state(ct, g)
+    # a dealiased state (one device check) lets the transposes carry the 2/3 box alone
+    p.flags |= resolve_flags(u_hat, g, None)
     return g, p, u_hat, ct
 
 

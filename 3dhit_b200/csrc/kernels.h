@@ -217,6 +217,8 @@ cudaError_t take_axis_timeout(int* flag);
 cudaError_t take_z_timeout(int* flag);
 cudaError_t set_axis_wait_limit(int polls);
 cudaError_t set_z_wait_limit(int polls);
+cudaError_t take_zadj_timeout(int* flag);
+cudaError_t set_zadj_wait_limit(int polls);
 template <typename T> int axis_tile_w(int N);
 
 // ---- reductions / elementwise (k_reduce.cu) ----------------------------------
@@ -280,6 +282,56 @@ struct AdjCoefArgs {
   int forcing;
   double ntot2, nu, A, eps, E_target, tau, tiny;
 };
+// Fused passes of the RHS transpose (k_xadj.cu, k_zadj.cu; columns with
+// xf_columns).  Cotangents are held in the padded general layout (3, Nx, Ny,
+// Mzp of the general geometry), states in the compact layout gs.
+template <typename T> struct AdjX1Args {
+  const V2<T>* u;    // state (3, gs.Mx, gs.My, gs.Mzp)
+  long long c_c, c_x;
+  const V2<T>* v;    // cotangent, entering as vscale v
+  long long v_c;
+  int v_p;           // its z pitch
+  T vscale;
+  V2<T>* t9;         // (9, Nx, gs.My, gs.Mzp): x-inverse of u, 1j k x u, project(dealias(v)) / w
+  long long t_c, t_x;
+  Geom gs;
+  KTab<T> k;
+  const V2<T>* tw;
+  T kmin2, kmax2;
+  double* partial;   // 6 per block: the sums of k_adj_sums
+};
+template <typename T> struct AdjX2Args {
+  const V2<T>* r6;   // (6, Nx, Ny, g.Mzp): y-forward of rfft(om x g), rfft(g x u)
+  const V2<T>* u;    // state (3, gs.Mx, gs.My, gs.Mzp)
+  long long c_c, c_x;
+  const V2<T>* v;    // cotangent of the RHS's value, entering as vscale v
+  const V2<T>* ubin; // cotangent of the step's result
+  V2<T>* acc;        // sum of the stages' cotangents so far
+  V2<T>* kb;         // the previous stage's v: c1 ubin + c2 sb
+  V2<T>* fb;         // nullable: sum of the stages' v (the held force's cotangent)
+  V2<T>* out;
+  int mode;          // 0: out = sb; 4: acc = ubin + sb, kb; 3, 2: acc += sb, kb; 1: out = acc + sb
+  int fb_first;
+  T vscale, c1, c2;
+  Geom g, gs;        // general geometry, geometry of the state
+  KTab<T> k;
+  const V2<T>* tw;
+  T nu, kmin2, kmax2;
+  const double* scal;
+};
+template <typename T> struct ZAdjArgs {
+  const V2<T>* in;   // (9, Nx, Ny, Mzp): x, y-physical u, om, g
+  V2<T>* out;        // (6, Nx, Ny, Mzpo): rfft of om x g, g x u
+  long long in_c, out_c;
+  int nrows, Mz, Mzp, Mzo, Mzpo;
+  T scale;           // 1 / (Nx Ny Nz)
+  const V2<T>* tw;
+};
+template <typename T> cudaError_t launch_adj_x1(const AdjX1Args<T>& a, int* nblocks, cudaStream_t st);
+template <typename T> cudaError_t launch_adj_x2(const AdjX2Args<T>& a, cudaStream_t st);
+template <typename T> cudaError_t launch_zadj(int H, const ZAdjArgs<T>& a, cudaStream_t st);
+// finalises the partials of k_adjx1 and forms the scalars (launch_adj_coef)
+cudaError_t launch_adj_scal(const double* partial, int nblocks, const AdjCoefArgs& a, cudaStream_t st);
 template <typename T> cudaError_t launch_adj_sums(const AdjArgs<T>& a, int nblocks, cudaStream_t st);
 cudaError_t launch_adj_coef(const AdjCoefArgs& a, cudaStream_t st);
 template <typename T> cudaError_t launch_adj_prep(const AdjArgs<T>& a, cudaStream_t st);

@@ -154,6 +154,10 @@ struct hit_plan {
   // transpose, its float64 sums and scalars, the RK4 stage inputs and
   // cotangents, and the rollout checkpoints
   Buf ax9, aph, as6, apart, asums, ascal, apct, ast[3], ak, akb, asb, aacc, aub, ack, aseg, afb;
+  // of the fused transpose (columns with xf_columns): x- and x,y-physical
+  // fields, products; cotangents in the padded general layout; stage inputs of
+  // one step, and of every step of a segment on the dealiased layout
+  Buf at9, au9, ar6, avb, avk, ava, avf, asg;
   cudaStream_t cap = nullptr;  // private stream used only for graph capture
   // side branch of the step for the forcing coefficient's reduction (see
   // fork_coef): its stream and one fork / join event pair per RK4 stage
@@ -282,11 +286,13 @@ template <typename T> int launch_coef(hit_plan* p, Path& P, const Scalars& s, in
   return HIT_OK;
 }
 
-// reference layout -> compact U (+ forcing coefficient of the gathered state)
-template <typename T> int gather_state(hit_plan* p, Path& P, const void* u_hat, const Scalars& s, cudaStream_t st) {
+// reference layout -> compact U, or dst (+ forcing coefficient of the gathered
+// state)
+template <typename T>
+int gather_state(hit_plan* p, Path& P, const void* u_hat, const Scalars& s, cudaStream_t st, V2<T>* dst = nullptr) {
   GatherArgs<T> a{};
   a.ext = static_cast<const V2<T>*>(u_hat);
-  a.cmp = vp<T>(P.U);
+  a.cmp = dst ? dst : vp<T>(P.U);
   a.g = P.g;
   a.k = ktab_of<T>(p);
   a.kmin2 = (T)s.kmin2;
@@ -1139,6 +1145,333 @@ int rollout_vjp_impl(hit_plan* p, const void* u0, const hit_params* pr, double d
   return HIT_OK;
 }
 
+// ---------------------------------------------------------------------------
+// fused transpose (columns with xf_columns): x passes of k_xadj.cu, z pass of
+// k_zadj.cu.  States in the compact layout of path P (the 2/3 box when the
+// caller states a dealiased state), cotangents in the padded general layout:
+// their modes outside the box stay nonzero.
+// ---------------------------------------------------------------------------
+
+// One stage: sb = (d rhs / d u)^T (vscale v) at the state u, then the algebra
+// `mode` of AdjX2Args on it; parameter cotangents added to pct.
+template <typename T> struct AdjStage {
+  const V2<T>* u;
+  const V2<T>* v;
+  T vscale;
+  int mode;
+  T c1, c2;
+  bool fb_first;
+};
+template <typename T>
+int adj_stage(hit_plan* p, Path& P, const Scalars& s, const AdjStage<T>& q, const V2<T>* ubin, V2<T>* acc, V2<T>* kb,
+              V2<T>* out, V2<T>* fb, double* pct, cudaStream_t st) {
+  const Geom& gs = P.g;
+  const Geom g = make_geom(p->Nx, p->Ny, p->Nz, false);
+  const size_t V = sizeof(V2<T>);
+  const long long t9c = (long long)g.Nx * gs.My * gs.Mzp, u9c = (long long)g.Nx * g.Ny * gs.Mzp;
+  const long long gc = (long long)g.Nx * g.Ny * g.Mzp;
+  int rc;
+  if ((rc = ensure(p->at9, 9 * t9c * V))) return rc;
+  if ((rc = ensure(p->au9, 9 * u9c * V))) return rc;
+  if ((rc = ensure(p->ar6, 6 * gc * V))) return rc;
+  if ((rc = ensure(p->apart, (size_t)6 * std::max(adj_blocks<T>(p), 64 * 148) * sizeof(double)))) return rc;
+  if ((rc = ensure(p->ascal, 8 * sizeof(double)))) return rc;
+  AdjX1Args<T> x{};
+  x.u = q.u;
+  x.c_c = (long long)gs.Mx * gs.My * gs.Mzp;
+  x.c_x = (long long)gs.My * gs.Mzp;
+  x.v = q.v;
+  x.v_c = gc;
+  x.v_p = g.Mzp;
+  x.vscale = q.vscale;
+  x.t9 = vp<T>(p->at9);
+  x.t_c = t9c;
+  x.t_x = (long long)gs.My * gs.Mzp;
+  x.gs = gs;
+  x.k = ktab_of<T>(p);
+  x.tw = tw_of<T>(p);
+  x.kmin2 = (T)s.kmin2;
+  x.kmax2 = (T)s.kmax2;
+  x.partial = static_cast<double*>(p->apart.p);
+  int nb = 0;
+  HIT_CK(launch_adj_x1<T>(x, &nb, st));
+  AdjCoefArgs c{};
+  c.scal = static_cast<double*>(p->ascal.p);
+  c.pct = pct;
+  c.forcing = s.forcing;
+  c.ntot2 = ntot2_of(p);
+  c.nu = s.nu;
+  c.A = s.A;
+  c.eps = s.eps;
+  c.E_target = s.E_target;
+  c.tau = s.tau;
+  c.tiny = tiny_of<T>();
+  HIT_CK(launch_adj_scal(x.partial, nb, c, st));
+  const int Wy = axis_tile_w<T>(g.Ny);
+  AxisArgs<T> a{};
+  a.src = vp<T>(p->at9);
+  a.dst = vp<T>(p->au9);
+  a.s_c = t9c;
+  a.s_a = gs.Mzp;
+  a.s_o = (long long)gs.My * gs.Mzp;
+  a.d_c = u9c;
+  a.d_a = gs.Mzp;
+  a.d_o = (long long)g.Ny * gs.Mzp;
+  a.Min = gs.My;
+  a.hin = gs.hy;
+  a.Mout = g.Ny;
+  a.hout = g.Ny / 2;
+  a.nz = gs.Mzp;
+  a.tw = tw_of<T>(p);
+  HIT_CK(launch_axis<T>(g.Ny, true, a, gs.Mzp / Wy, g.Nx, 9, st));
+  ZAdjArgs<T> z{};
+  z.in = vp<T>(p->au9);
+  z.out = vp<T>(p->ar6);
+  z.in_c = u9c;
+  z.out_c = gc;
+  z.nrows = g.Nx * g.Ny;
+  z.Mz = gs.Mz;
+  z.Mzp = gs.Mzp;
+  z.Mzo = g.Mz;
+  z.Mzpo = g.Mzp;
+  z.scale = (T)(1.0 / ((double)g.Nx * g.Ny * g.Nz));
+  z.tw = tw_of<T>(p);
+  HIT_CK(launch_zadj<T>(g.H, z, st));
+  AxisArgs<T> b{};
+  b.src = b.dst = vp<T>(p->ar6);
+  b.s_c = b.d_c = gc;
+  b.s_a = b.d_a = g.Mzp;
+  b.s_o = b.d_o = (long long)g.Ny * g.Mzp;
+  b.Min = b.Mout = g.Ny;
+  b.hin = b.hout = g.Ny / 2;
+  b.nz = g.Mzp;
+  b.tw = tw_of<T>(p);
+  HIT_CK(launch_axis<T>(g.Ny, false, b, g.Mzp / Wy, g.Nx, 6, st));
+  AdjX2Args<T> y{};
+  y.r6 = vp<T>(p->ar6);
+  y.u = q.u;
+  y.c_c = x.c_c;
+  y.c_x = x.c_x;
+  y.v = q.v;
+  y.ubin = ubin;
+  y.acc = acc;
+  y.kb = kb;
+  y.fb = fb;
+  y.out = out;
+  y.mode = q.mode;
+  y.fb_first = q.fb_first ? 1 : 0;
+  y.vscale = q.vscale;
+  y.c1 = q.c1;
+  y.c2 = q.c2;
+  y.g = g;
+  y.gs = gs;
+  y.k = ktab_of<T>(p);
+  y.tw = tw_of<T>(p);
+  y.nu = (T)s.nu;
+  y.kmin2 = (T)s.kmin2;
+  y.kmax2 = (T)s.kmax2;
+  y.scal = static_cast<const double*>(p->ascal.p);
+  HIT_CK(launch_adj_x2<T>(y, st));
+  return HIT_OK;
+}
+
+// Stage inputs of one RK4 step from the compact state u (integrators.py:32-38):
+// S[0..2] receive those of stages 2..4 and, when u_next is given, u_next the
+// new state.  x_ready: the x-inverse of u is in P.t6 already (left by the
+// previous step's stage 4); P.coef holds u's forcing coefficient.
+template <typename T>
+int adj_forward(hit_plan* p, Path& P, const Scalars& s, double dt, V2<T>* u, V2<T>* const (&S)[3], V2<T>* u_next,
+                bool x_ready, const V2<T>* fext, cudaStream_t st) {
+  int rc;
+  const bool red = needs_coef(s.forcing);
+  if (!x_ready && (rc = launch_p1_of<T>(p, P, u, st))) return rc;
+  const int last = u_next ? 4 : 3;
+  for (int stage = 1; stage <= last; ++stage) {
+    if ((rc = launch_p2<T>(p, P, st))) return rc;
+    if (red && stage > 1 && (rc = join_coef(p, stage - 2, st))) return rc;
+    StageBufs<T> b;
+    b.u = u;
+    b.s_in = stage > 1 ? S[stage - 2] : u;
+    b.s_out = stage < 4 ? S[stage - 1] : S[2];
+    b.u_out = u_next;
+    const bool fuse = stage < last || u_next;
+    if ((rc = launch_p3_stage<T>(p, P, s, stage, dt, fuse, red && fuse, fext, st, false, false, b))) return rc;
+    if (red && fuse && (rc = fork_coef<T>(p, P, s, stage - 1, st))) return rc;
+  }
+  if (red && u_next && (rc = join_coef(p, 3, st))) return rc;
+  return HIT_OK;
+}
+
+// vub = (d rk4_step / d u)^T vub with the step's stage inputs in u[0..3]
+// (fb: see AdjX2Args).
+template <typename T>
+int adj_step(hit_plan* p, Path& P, const Scalars& s, double dt, const V2<T>* const (&u)[4], V2<T>* vub, V2<T>* fb,
+             double* pct, cudaStream_t st) {
+  const long long gc = (long long)p->Nx * p->Ny * make_geom(p->Nx, p->Ny, p->Nz, false).Mzp;
+  int rc;
+  if ((rc = ensure(p->avk, 3 * gc * sizeof(V2<T>)))) return rc;
+  if ((rc = ensure(p->ava, 3 * gc * sizeof(V2<T>)))) return rc;
+  V2<T>* kb = vp<T>(p->avk);
+  V2<T>* acc = vp<T>(p->ava);
+  const T h = (T)(0.5 * dt), d = (T)dt, d3 = (T)(dt / 3.0), d6 = (T)(dt / 6.0);
+  // transpose of u + dt/6 (k1 + 2 k2 + 2 k3 + k4), stage by stage backwards
+  const AdjStage<T> q[4] = {{u[3], vub, d6, 4, d3, d, true},
+                            {u[2], kb, T(1), 3, d3, h, false},
+                            {u[1], kb, T(1), 2, d6, h, false},
+                            {u[0], kb, T(1), 1, T(0), T(0), false}};
+  for (const AdjStage<T>& a : q)
+    if ((rc = adj_stage<T>(p, P, s, a, vub, acc, kb, vub, fb, pct, st))) return rc;
+  return HIT_OK;
+}
+
+// reference layout <-> padded general layout of a cotangent
+template <typename T> int gather_cotangent(hit_plan* p, const void* v, V2<T>* dst, cudaStream_t st) {
+  GatherArgs<T> a{};
+  a.ext = static_cast<const V2<T>*>(v);
+  a.cmp = dst;
+  a.g = make_geom(p->Nx, p->Ny, p->Nz, false);
+  a.k = ktab_of<T>(p);
+  HIT_CK(launch_gather<T>(a, adj_blocks<T>(p), st));
+  return HIT_OK;
+}
+template <typename T> int scatter_cotangent(hit_plan* p, const V2<T>* v, void* dst, cudaStream_t st) {
+  HIT_CK(launch_scatter<T>(v, static_cast<V2<T>*>(dst), make_geom(p->Nx, p->Ny, p->Nz, false), st));
+  return HIT_OK;
+}
+template <typename T> size_t cotangent_bytes(const hit_plan* p) {
+  return (size_t)3 * p->Nx * p->Ny * make_geom(p->Nx, p->Ny, p->Nz, false).Mzp * sizeof(V2<T>);
+}
+
+// The stage inputs of one step as compact states: u gathered into P.U, S2..S4
+// in p->ast.
+template <typename T>
+int adj_states(hit_plan* p, Path& P, const Scalars& s, double dt, const void* u, const V2<T>* fext,
+               const V2<T>* (&out)[4], cudaStream_t st) {
+  const size_t cmp = (size_t)3 * P.g.Mx * P.g.My * P.g.Mzp * sizeof(V2<T>);
+  int rc;
+  for (Buf& b : p->ast)
+    if ((rc = ensure(b, cmp))) return rc;
+  V2<T>* S[3] = {vp<T>(p->ast[0]), vp<T>(p->ast[1]), vp<T>(p->ast[2])};
+  if ((rc = gather_state<T>(p, P, u, s, st))) return rc;
+  if ((rc = adj_forward<T>(p, P, s, dt, vp<T>(P.U), S, nullptr, false, fext, st))) return rc;
+  out[0] = vp<T>(P.U);
+  for (int i = 0; i < 3; ++i) out[i + 1] = S[i];
+  return HIT_OK;
+}
+
+template <typename T>
+int rhs_vjp_fused(hit_plan* p, const void* u, const hit_params* pr, const void* v, void* ub, double* pct,
+                  cudaStream_t st) {
+  const int which = (pr->flags & HIT_FLAG_ASSUME_DEALIASED) ? 1 : 0;
+  int rc;
+  if ((rc = ensure_path<T>(p, which))) return rc;
+  Path& P = p->path[which];
+  Scalars s = scalars_of(pr);
+  if ((rc = ensure(p->avb, cotangent_bytes<T>(p)))) return rc;
+  if ((rc = ensure(p->avk, cotangent_bytes<T>(p)))) return rc;
+  Scalars plain = s;
+  plain.forcing = 0;  // no coefficient needed: the transpose forms its own sums
+  if ((rc = gather_state<T>(p, P, u, plain, st))) return rc;
+  if ((rc = gather_cotangent<T>(p, v, vp<T>(p->avb), st))) return rc;
+  const AdjStage<T> q{vp<T>(P.U), vp<T>(p->avb), T(1), 0, T(0), T(0), false};
+  if ((rc = adj_stage<T>(p, P, s, q, nullptr, nullptr, nullptr, vp<T>(p->avk), nullptr, pct, st))) return rc;
+  return scatter_cotangent<T>(p, vp<T>(p->avk), ub, st);
+}
+
+template <typename T>
+int rk4_vjp_fused(hit_plan* p, const void* u, const hit_params* pr, double dt, const void* ub_in, void* ub_out,
+                  double* pct, cudaStream_t st, const void* fext = nullptr, V2<T>* fbar = nullptr) {
+  const int which = (pr->flags & HIT_FLAG_ASSUME_DEALIASED) ? 1 : 0;
+  int rc;
+  if ((rc = ensure_path<T>(p, which))) return rc;
+  Path& P = p->path[which];
+  const Scalars s = scalars_of(pr);
+  if ((rc = ensure(p->avb, cotangent_bytes<T>(p)))) return rc;
+  V2<T>* FB = nullptr;
+  if (fbar) {
+    if ((rc = ensure(p->avf, cotangent_bytes<T>(p)))) return rc;
+    FB = vp<T>(p->avf);
+  }
+  if (fext && (rc = gather_force<T>(p, P, fext, st))) return rc;
+  const V2<T>* states[4];
+  if ((rc = adj_states<T>(p, P, s, dt, u, fext ? vp<T>(P.FEXT) : nullptr, states, st))) return rc;
+  if ((rc = gather_cotangent<T>(p, ub_in, vp<T>(p->avb), st))) return rc;
+  if ((rc = adj_step<T>(p, P, s, dt, states, vp<T>(p->avb), FB, pct, st))) return rc;
+  if ((rc = scatter_cotangent<T>(p, vp<T>(p->avb), ub_out, st))) return rc;
+  if (fbar) {  // every stage adds P f: fbar = P (sum of the stages' cotangents)
+    const Geom g = make_geom(p->Nx, p->Ny, p->Nz, false);
+    if ((rc = ensure(p->afb, (size_t)3 * g.Nx * g.Ny * g.Nzh * sizeof(V2<T>)))) return rc;
+    if ((rc = scatter_cotangent<T>(p, FB, p->afb.p, st))) return rc;
+    HIT_CK(launch_dealias_project<T>(vp<T>(p->afb), fbar, g, ktab_of<T>(p), 1, 1, st));
+  }
+  return HIT_OK;
+}
+
+// u0_bar = (d rollout / d u0)^T ub: states every K steps are kept (reference
+// layout), each segment is run forwards again and transposed step by step.  On
+// the dealiased layout a compact state is a third of a full one, and the
+// segment keeps all four stage inputs of its steps, so nothing is recomputed
+// twice; on the general layout it keeps the steps' states and recomputes the
+// stage inputs.
+template <typename T>
+int rollout_vjp_fused(hit_plan* p, const void* u0, const hit_params* pr, double dt, int64_t nsteps, int K,
+                      const void* ub, void* u0_bar, double* pct, cudaStream_t st) {
+  const int which = (pr->flags & HIT_FLAG_ASSUME_DEALIASED) ? 1 : 0;
+  const long long n = 3LL * p->Nx * p->Ny * (p->Nz / 2 + 1);
+  const size_t bytes = n * sizeof(V2<T>);
+  const int64_t nseg = (nsteps + K - 1) / K;
+  int rc;
+  if (nsteps == 0) {
+    HIT_CK(cudaMemcpyAsync(u0_bar, ub, bytes, cudaMemcpyDeviceToDevice, st));
+    return HIT_OK;
+  }
+  if ((rc = ensure_path<T>(p, which))) return rc;
+  Path& P = p->path[which];
+  const Scalars s = scalars_of(pr);
+  const long long cmp = 3LL * P.g.Mx * P.g.My * P.g.Mzp;
+  if ((rc = ensure(p->ack, nseg * bytes))) return rc;
+  if ((rc = ensure(p->avb, cotangent_bytes<T>(p)))) return rc;
+  if (which) {
+    if ((rc = ensure(p->asg, (size_t)4 * K * cmp * sizeof(V2<T>)))) return rc;
+  } else {
+    if ((rc = ensure(p->aseg, (size_t)K * bytes))) return rc;
+  }
+  V2<T>* CK = vp<T>(p->ack);
+  V2<T>* VB = vp<T>(p->avb);
+  if ((rc = gather_cotangent<T>(p, ub, VB, st))) return rc;
+  HIT_CK(cudaMemcpyAsync(CK, u0, bytes, cudaMemcpyDeviceToDevice, st));
+  for (int64_t j = 1; j < nseg; ++j)
+    if ((rc = rollout_impl<T>(p, CK + (j - 1) * n, pr, dt, K, CK + j * n, nullptr, st))) return rc;
+  for (int64_t j = nseg - 1; j >= 0; --j) {
+    const int len = (int)std::min<int64_t>(K, nsteps - j * K);
+    if (which) {
+      V2<T>* A = vp<T>(p->asg);
+      if ((rc = gather_state<T>(p, P, CK + j * n, s, st, A))) return rc;
+      for (int i = 0; i < len; ++i) {
+        V2<T>* u = A + 4LL * i * cmp;
+        V2<T>* S[3] = {u + cmp, u + 2 * cmp, u + 3 * cmp};
+        if ((rc = adj_forward<T>(p, P, s, dt, u, S, i + 1 < len ? u + 4 * cmp : nullptr, i > 0, nullptr, st))) return rc;
+      }
+      for (int i = len - 1; i >= 0; --i) {
+        const V2<T>* u = A + 4LL * i * cmp;
+        const V2<T>* states[4] = {u, u + cmp, u + 2 * cmp, u + 3 * cmp};
+        if ((rc = adj_step<T>(p, P, s, dt, states, VB, nullptr, pct, st))) return rc;
+      }
+    } else {
+      V2<T>* SEG = vp<T>(p->aseg);
+      HIT_CK(cudaMemcpyAsync(SEG, CK + j * n, bytes, cudaMemcpyDeviceToDevice, st));
+      for (int i = 1; i < len; ++i)
+        if ((rc = rollout_impl<T>(p, SEG + (i - 1) * n, pr, dt, 1, SEG + i * n, nullptr, st))) return rc;
+      for (int i = len - 1; i >= 0; --i) {
+        const V2<T>* states[4];
+        if ((rc = adj_states<T>(p, P, s, dt, SEG + i * n, nullptr, states, st))) return rc;
+        if ((rc = adj_step<T>(p, P, s, dt, states, VB, nullptr, pct, st))) return rc;
+      }
+    }
+  }
+  return scatter_cotangent<T>(p, VB, u0_bar, st);
+}
+
 // entry-point wrappers: zero the parameter cotangents, run, copy them out
 template <typename T>
 int vjp_entry(hit_plan* p, int which, const void* u, const hit_params* pr, double dt, int64_t nsteps, int K,
@@ -1150,7 +1483,11 @@ int vjp_entry(hit_plan* p, int which, const void* u, const hit_params* pr, doubl
   const V2<T>* uu = static_cast<const V2<T>*>(u);
   const V2<T>* cc = static_cast<const V2<T>*>(ct);
   V2<T>* ub = static_cast<V2<T>*>(ubar);
-  if (which == 0) rc = rhs_vjp_impl<T>(p, uu, scalars_of(pr), cc, ub, pct, st);
+  if (xf_columns<T>(p->Nx)) {
+    if (which == 0) rc = rhs_vjp_fused<T>(p, u, pr, ct, ubar, pct, st);
+    else if (which == 1) rc = rk4_vjp_fused<T>(p, u, pr, dt, ct, ubar, pct, st);
+    else rc = rollout_vjp_fused<T>(p, u, pr, dt, nsteps, K, ct, ubar, pct, st);
+  } else if (which == 0) rc = rhs_vjp_impl<T>(p, uu, scalars_of(pr), cc, ub, pct, st);
   else if (which == 1) rc = rk4_vjp_impl<T>(p, uu, pr, dt, cc, ub, pct, st);
   else rc = rollout_vjp_impl<T>(p, u, pr, dt, nsteps, K, ct, ubar, pct, st);
   if (rc) return rc;
@@ -1165,9 +1502,11 @@ int forced_vjp_entry(hit_plan* p, const void* u, const hit_params* pr, const voi
   if ((rc = ensure(p->apct, 4 * sizeof(double)))) return rc;
   double* pct = static_cast<double*>(p->apct.p);
   HIT_CK(cudaMemsetAsync(pct, 0, 4 * sizeof(double), st));
-  if ((rc = rk4_vjp_impl<T>(p, static_cast<const V2<T>*>(u), pr, dt, static_cast<const V2<T>*>(ct),
-                            static_cast<V2<T>*>(ubar), pct, st, f, static_cast<V2<T>*>(fbar))))
-    return rc;
+  rc = xf_columns<T>(p->Nx)
+           ? rk4_vjp_fused<T>(p, u, pr, dt, ct, ubar, pct, st, f, static_cast<V2<T>*>(fbar))
+           : rk4_vjp_impl<T>(p, static_cast<const V2<T>*>(u), pr, dt, static_cast<const V2<T>*>(ct),
+                             static_cast<V2<T>*>(ubar), pct, st, f, static_cast<V2<T>*>(fbar));
+  if (rc) return rc;
   if (pct_out) HIT_CK(cudaMemcpyAsync(pct_out, pct, 3 * sizeof(double), cudaMemcpyDeviceToDevice, st));
   return HIT_OK;
 }
@@ -1322,7 +1661,8 @@ int hit_plan_destroy(hit_plan* p) {
   release(p->dpartial);
   release(p->dsums);
   for (Buf* b : {&p->ax9, &p->aph, &p->as6, &p->apart, &p->asums, &p->ascal, &p->apct, &p->ast[0], &p->ast[1],
-                 &p->ast[2], &p->ak, &p->akb, &p->asb, &p->aacc, &p->aub, &p->ack, &p->aseg, &p->afb})
+                 &p->ast[2], &p->ak, &p->akb, &p->asb, &p->aacc, &p->aub, &p->ack, &p->aseg, &p->afb, &p->at9,
+                 &p->au9, &p->ar6, &p->avb, &p->avk, &p->ava, &p->avf, &p->asg})
     release(*b);
   if (p->cap) cudaStreamDestroy(p->cap);
   if (p->side) cudaStreamDestroy(p->side);
@@ -1405,14 +1745,17 @@ int hit_device_status(int* status) {
   int z = 0;
   cudaError_t e = take_axis_timeout(status);
   if (e == cudaSuccess) e = take_z_timeout(&z);
+  int za = 0;
+  if (e == cudaSuccess) e = take_zadj_timeout(&za);
   if (e != cudaSuccess) return cuda_fail(e, "device_status");
-  *status = *status || z;
+  *status = *status || z || za;
   return HIT_OK;
 }
 
 int hit_set_wait_limit(int polls) {
   cudaError_t e = set_axis_wait_limit(polls);
   if (e == cudaSuccess) e = set_z_wait_limit(polls);
+  if (e == cudaSuccess) e = set_zadj_wait_limit(polls);
   return e == cudaSuccess ? HIT_OK : cuda_fail(e, "set_wait_limit");
 }
 
