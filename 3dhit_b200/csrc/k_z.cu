@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(NWARP * 32, ZW_MINB) k_zwarp(ZCrossArgs<float>
   auto below = [](int k, int lo, int hi, int bound) { return hi < bound ? true : (lo >= bound ? false : k < bound); };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = lane / Z::LPR, b = lane % Z::LPR;
-  const ZwMid<H> mid(b);
+  ZwMid<H> mid(b);
   float2 wl[7];  // filled once the twiddle tables are in shared memory
   const int stg_slots = 6 * Z::ROWS * Mzp;
   float2* stg = tws + Z::TWS + warp * (stg_slots + Z::ROWS * Z::XS);  // [field][row][Mzp]
@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(NWARP * 32, ZW_MINB) k_zwarp(ZCrossArgs<float>
   tma::fence_async_smem();
   __syncthreads();
   zw_last_twiddles<H>(wl, tws, b);
+  mid.load(tws);
 
   const int wait_limit = g_z_wait_limit;
   const long long ngroups = a.nrows / Z::ROWS;
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(ZP_WARPS * 32, ZW_MINB) k_zpair(ZCrossArgs<flo
   auto below = [](int k, int lo, int hi, int bound) { return hi < bound ? true : (lo >= bound ? false : k < bound); };
   const int team = threadIdx.x >> 6, b = threadIdx.x & 63, lane = threadIdx.x & 31;
   const int bar_id = 1 + team;
-  const ZwMid<H> mid(b);
+  ZwMid<H> mid(b);
   float2 wl[7];  // filled once the twiddle tables are in shared memory
   const int stg_slots = 6 * Mzp;
   float2* stg = tws + Z::TWS + team * (stg_slots + Z::XS);  // [field][Mzp]
@@ -506,6 +507,7 @@ __global__ void __launch_bounds__(ZP_WARPS * 32, ZW_MINB) k_zpair(ZCrossArgs<flo
   tma::fence_async_smem();
   __syncthreads();
   zw_last_twiddles<H>(wl, tws, b);
+  mid.load(tws);
 
   const int wait_limit = g_z_wait_limit;
   const long long nteams = (long long)gridDim.x * NTEAM;

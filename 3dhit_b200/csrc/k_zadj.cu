@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(ZA_WARPS * 32, ZA_MINB) k_zadjw(ZAdjArgs<float
   auto below = [](int k, int lo, int hi, int bound) { return hi < bound ? true : (lo >= bound ? false : k < bound); };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = lane / Z::LPR, b = lane % Z::LPR;
-  const ZwMid<H> mid(b);
+  ZwMid<H> mid(b);
   float2 wl[7];
   const int stg_slots = 9 * Z::ROWS * Mzp;
   float2* stg = tws + Z::TWS + warp * (stg_slots + Z::ROWS * Z::XS);  // [field][row][Mzp]
@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(ZA_WARPS * 32, ZA_MINB) k_zadjw(ZAdjArgs<float
   tma::fence_async_smem();
   __syncthreads();
   zw_last_twiddles<H>(wl, tws, b);
+  mid.load(tws);
   const int wait_limit = g_zadj_wait_limit;
   const long long ngroups = a.nrows / Z::ROWS;
   const long long nwarps = (long long)gridDim.x * ZA_WARPS;

@@ -129,6 +129,13 @@ template <int H> struct ZwMid {
   int k[C1];   // twiddle index b1 % 8
   int ld[C1];  // exchange slot of input b1 (input r at ld + zw_slot(r H / R1))
   int st[C1];  // exchange slot of output j (output r at st + zw_slot(8 r))
+  float2 w[C1][R1 > 1 ? R1 - 1 : 1];
+  __device__ __forceinline__ void load(const float2* tws) {
+#pragma unroll
+    for (int i = 0; i < C1; ++i)
+#pragma unroll
+      for (int r = 1; r < R1; ++r) w[i][r - 1] = tws[ZW<H>::TW1 + (r - 1) * 8 + k[i]];
+  }
   // once per thread (a load of the table at H = 256, 512).  The offsets are
   // additive: H / R1 = 64 is a multiple of 16, and j % 16 = b1 % 8 leaves
   // room for 8 r % 16 below 16.
@@ -199,10 +206,9 @@ __device__ __forceinline__ void zw_transform(float2 (&v)[8], float2* xch, const 
     zw_sync<H>(bar_id);
 #pragma unroll
     for (int i = 0; i < C1; ++i) {
-      const int k = mid.k[i];
 #pragma unroll
       for (int r = 1; r < R1; ++r) {
-        float2 w = tws[Z::TW1 + (r - 1) * 8 + k];
+        float2 w = mid.w[i][r - 1];
         if (INV) w.y = -w.y;
         u[i][r] = cmul(u[i][r], w);
       }
