@@ -126,6 +126,18 @@ template <typename T> struct ZCrossArgs {
   const V2<T>* tw;
 };
 
+// Middle of the RHS on planes that fit in shared memory (k_plane.cu): T6 in
+// place, fields 0..5 in, the products in fields 0..2 out.
+template <typename T> struct PlaneArgs {
+  V2<T>* t6;  // (6, Nx, My, Mzp)
+  long long t_c, t_x;
+  Geom g;
+  T scale;    // 1/(Nx Ny Nz)
+  const V2<T>* tw;
+};
+bool plane_fits(const Geom& g);
+template <typename T> cudaError_t launch_plane(const PlaneArgs<T>& a, cudaStream_t st);
+
 // z pass of the fused LES stage (k_zles, float32): per (x, y) row, c2r of u
 // and the nine velocity gradients, u x w and the closure MLP per physical
 // point, r2c of the three products and the six SGS stresses (xx, yy, zz,
@@ -218,6 +230,8 @@ cudaError_t take_z_timeout(int* flag);
 cudaError_t set_axis_wait_limit(int polls);
 cudaError_t set_z_wait_limit(int polls);
 cudaError_t take_zadj_timeout(int* flag);
+cudaError_t take_plane_timeout(int* flag);
+cudaError_t set_plane_wait_limit(int polls);
 cudaError_t set_zadj_wait_limit(int polls);
 template <typename T> int axis_tile_w(int N);
 

@@ -320,10 +320,22 @@ template <typename T> int launch_p1_of(hit_plan* p, Path& P, const V2<T>* src, c
   return HIT_OK;
 }
 
-// P2a, P2b, P2c: T6 -> U6 (y-inverse), z pass in place on U6, U6[0:3] -> T6[0:3]
+// P2a, P2b, P2c: T6 -> U6 (y-inverse), z pass in place on U6, U6[0:3] -> T6[0:3];
+// one kernel over T6 in place where the planes fit in shared memory
 template <typename T> int launch_p2(hit_plan* p, Path& P, cudaStream_t st, Prof* pf = nullptr) {
   const Geom& g = P.g;
   const long long t6c = (long long)g.Nx * g.My * g.Mzp, u6c = (long long)g.Nx * g.Ny * g.Mzp;
+  if (plane_fits(g)) {
+    PlaneArgs<T> q{};
+    q.t6 = vp<T>(P.t6);
+    q.t_c = t6c;
+    q.t_x = (long long)g.My * g.Mzp;
+    q.g = g;
+    q.scale = (T)(1.0 / ((double)g.Nx * g.Ny * g.Nz));
+    q.tw = tw_of<T>(p);
+    TIMED(pf, 2, ck(launch_plane<T>(q, st), "plane pass"));
+    return HIT_OK;
+  }
   const int Wy = axis_tile_w<T>(g.Ny);
   AxisArgs<T> a{};
   a.src = vp<T>(P.t6);
@@ -1745,10 +1757,11 @@ int hit_device_status(int* status) {
   int z = 0;
   cudaError_t e = take_axis_timeout(status);
   if (e == cudaSuccess) e = take_z_timeout(&z);
-  int za = 0;
+  int za = 0, zp = 0;
   if (e == cudaSuccess) e = take_zadj_timeout(&za);
+  if (e == cudaSuccess) e = take_plane_timeout(&zp);
   if (e != cudaSuccess) return cuda_fail(e, "device_status");
-  *status = *status || z || za;
+  *status = *status || z || za || zp;
   return HIT_OK;
 }
 
@@ -1756,6 +1769,7 @@ int hit_set_wait_limit(int polls) {
   cudaError_t e = set_axis_wait_limit(polls);
   if (e == cudaSuccess) e = set_z_wait_limit(polls);
   if (e == cudaSuccess) e = set_zadj_wait_limit(polls);
+  if (e == cudaSuccess) e = set_plane_wait_limit(polls);
   return e == cudaSuccess ? HIT_OK : cuda_fail(e, "set_wait_limit");
 }
 
