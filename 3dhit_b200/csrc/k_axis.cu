@@ -935,6 +935,17 @@ template <typename F> cudaError_t dispatch_len(int N, F&& f) {
   }
 }
 
+// lengths that k_axis serves (the column passes of shorter ones are k_col's)
+template <typename F> cudaError_t dispatch_long(int N, F&& f) {
+  switch (N) {
+    case 128: return f(std::integral_constant<int, 128>{});
+    case 256: return f(std::integral_constant<int, 256>{});
+    case 512: return f(std::integral_constant<int, 512>{});
+    case 1024: return f(std::integral_constant<int, 1024>{});
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 // P1 shared memory: A, B, the twiddles and the 3 staged components (N x W
 // each); P3: A, B, the staged nl column (N x W), the twiddles and, in
 // shared-memory mode, the 3 compact tiles (Mx x W).  (Twiddle slots rounded to
@@ -996,16 +1007,18 @@ bool axis_map(CUtensorMap* m, const V2<T>* base, long long cols, int rows, int n
 
 template <typename T>
 cudaError_t launch_axis(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, int nc, cudaStream_t st) {
-  return dispatch_len(N, [&](auto nn) {
+  // staging needs 16-byte aligned rows and whole tiles inside the source rows
+  // (which may extend past the nz valid columns: padded rows)
+  const long long cols = a.src_cols > 0 ? a.src_cols : a.nz;
+  const bool pf = (sizeof(V2<T>) == 16 || ((a.s_a | a.s_o | a.s_c) % 2 == 0 && ((uintptr_t)a.src % 16) == 0)) &&
+                  (long long)nzt * tile_w<T>(N) <= cols;
+  const long long ntiles = (long long)nzt * no * nc;
+  if (col_pass<T>(N, inv, pf, ntiles * N * tile_w<T>(N) * (long long)sizeof(V2<T>)))
+    return launch_col<T>(N, inv, a, nzt, no, nc, st);
+  return dispatch_long(N, [&](auto nn) {
     constexpr int NN = decltype(nn)::value;
     constexpr int W = tile_w<T>(NN);
-    const long long ntiles = (long long)nzt * no * nc;
     if ((inv ? a.Mout : a.Min) != NN) return cudaErrorInvalidValue;  // the full side is all N rows
-    // staging needs 16-byte aligned rows and whole tiles inside the source rows
-    // (which may extend past the nz valid columns: padded rows)
-    const bool pf = (sizeof(V2<T>) == 16 || ((a.s_a | a.s_o | a.s_c) % 2 == 0 &&
-                                              ((uintptr_t)a.src % 16) == 0)) &&
-                    (long long)nzt * W <= (a.src_cols > 0 ? a.src_cols : a.nz);
     static PerDevice c[6];
     CUtensorMap mA{}, mB{};
     if (pf) {
@@ -1018,7 +1031,6 @@ cudaError_t launch_axis(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, 
       while (t.br > 2 && t.br * (nb(a.hin, t.br) + nb(t.pb, t.br)) > NN) t.br /= 2;
       t.ka = nb(a.hin, t.br);
       t.kb = nb(t.pb, t.br);
-      const long long cols = a.src_cols > 0 ? a.src_cols : a.nz;
       const bool tma = a.hin >= 1 && t.pb >= 1 && t.br * (t.ka + t.kb) <= NN && ((uintptr_t)a.src % 16) == 0 &&
                        axis_map<T>(&mA, a.src, cols, a.hin, no, nc, a.s_a, a.s_o, a.s_c, W, t.br) &&
                        axis_map<T>(&mB, a.src + (long long)a.hin * a.s_a, cols, t.pb, no, nc, a.s_a, a.s_o, a.s_c, W,
@@ -1036,7 +1048,8 @@ cudaError_t launch_axis(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, 
                           NT, smem, st, a, nzt, no, (int)ntiles, mA, mB);
       return launch_pdl(k_axis<T, NN, W, false, 1>, resident_grid(k_axis<T, NN, W, false, 1>, NT, smem, ntiles, c[1]),
                         NT, smem, st, a, nzt, no, (int)ntiles, mA, mB);
-    } else {
+    }
+    if constexpr (NN > 256) {
       const size_t smem = axis_smem<T, NN, W, false>();
       if (inv)
         k_axis<T, NN, W, true, 0><<<resident_grid(k_axis<T, NN, W, true, 0>, NT, smem, ntiles, c[2]), NT, smem, st>>>(
@@ -1044,8 +1057,9 @@ cudaError_t launch_axis(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, 
       else
         k_axis<T, NN, W, false, 0><<<resident_grid(k_axis<T, NN, W, false, 0>, NT, smem, ntiles, c[3]), NT, smem,
                                      st>>>(a, nzt, no, (int)ntiles, mA, mB);
+      return cudaGetLastError();
     }
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;  // unaligned rows of shorter columns: k_col
   });
 }
 
@@ -1202,7 +1216,8 @@ template <typename T> cudaError_t launch_p3(const P3Args<T>& a, cudaStream_t st)
 }
 
 template <typename T> cudaError_t prepare_axis_kernels(int Nx) {
-  return dispatch_len(Nx, [&](auto nn) {
+  if (Nx < 128) return cudaSuccess;
+  return dispatch_long(Nx, [&](auto nn) {
     constexpr int NN = decltype(nn)::value;
     cudaError_t e;
     constexpr int W = tile_w<T>(NN);
@@ -1210,8 +1225,11 @@ template <typename T> cudaError_t prepare_axis_kernels(int Nx) {
     if ((e = max_smem(k_axis<T, NN, W, false, 2>, (int)axis_smem<T, NN, W, true>())) != cudaSuccess) return e;
     if ((e = max_smem(k_axis<T, NN, W, true, 1>, (int)axis_smem<T, NN, W, true>())) != cudaSuccess) return e;
     if ((e = max_smem(k_axis<T, NN, W, false, 1>, (int)axis_smem<T, NN, W, true>())) != cudaSuccess) return e;
-    if ((e = max_smem(k_axis<T, NN, W, true, 0>, (int)axis_smem<T, NN, W, false>())) != cudaSuccess) return e;
-    return max_smem(k_axis<T, NN, W, false, 0>, (int)axis_smem<T, NN, W, false>());
+    if constexpr (NN > 256) {
+      if ((e = max_smem(k_axis<T, NN, W, true, 0>, (int)axis_smem<T, NN, W, false>())) != cudaSuccess) return e;
+      return max_smem(k_axis<T, NN, W, false, 0>, (int)axis_smem<T, NN, W, false>());
+    }
+    return cudaSuccess;
   });
 }
 

@@ -856,12 +856,12 @@ template <typename T> cudaError_t launch_zcross(int H, const ZCrossArgs<T>& a, c
     // Rows per CTA group.  float64 takes half the rows of float32: its groups
     // fill 110 KB otherwise, two CTAs (six warps) per SM (z pass 82 -> 62 us at
     // 128^3, 580 -> 408 at 256^3; a quarter: 83 and 678).  Grids with few rows
-    // take a sixteenth, so that every SM has groups (32 x 32 rows of 32 points
-    // in groups of 32 ran on 32 CTAs: 18.9 us; in groups of 2: 8.5; 64^3 float64
-    // step 153 -> 142 us).
+    // take a sixteenth, at least two, so that every SM has groups (32 x 32 rows
+    // of 32 points in groups of 32 ran on 32 CTAs: 18.9 us; in groups of 2: 8.5;
+    // 64^3 float64 general layout in groups of 1: 26, 2: 19, 16: 21).
     constexpr int RB0 = z_rows_per_block<HH>();
     constexpr int RB = sizeof(T) == 8 && RB0 > 1 ? RB0 / 2 : RB0;
-    constexpr int RS = RB0 / 16 < 1 ? 1 : RB0 / 16;
+    constexpr int RS = RB0 >= 32 ? RB0 / 16 : (RB0 < 2 ? RB0 : 2);
     if (RS < RB && a.nrows < 4 * 148 * RB) return launch_zcross_v<T, HH, RS, z_threads<HH>(), 4>(a, st);
     return launch_zcross_v<T, HH, RB, z_threads<HH>(), 4>(a, st);
   });
@@ -919,29 +919,43 @@ cudaError_t launch_zles(int H, const ZLesArgs& a, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
-template <typename T, bool C2R> cudaError_t launch_zreal(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st) {
+// Rows whose length the warp-resident kernels take have no CTA-per-group form.
+template <typename T, int H> constexpr bool zreal_cta() { return sizeof(T) == 8 || !zrealw_length(H); }
+
+template <typename T> cudaError_t launch_zc2r(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (zrealw_length(H)) return zrealw_ok(H, a) ? launch_zc2rw(H, a, ncomp, st) : cudaErrorInvalidValue;
+  }
   if (a.Mzp % 8 || ((uintptr_t)a.cbuf % 16) || ((uintptr_t)a.rbuf % 16)) return cudaErrorInvalidValue;
   return dispatch_half(H, [&](auto hh) {
     constexpr int HH = decltype(hh)::value;
     constexpr int RB = z_rows_per_block<HH>(), NTZ = z_threads<HH>();
-    if (a.Mzp > z_row_cap<HH>()) return cudaErrorInvalidValue;
-    static PerDevice cache;
-    const long long work = (a.nrows + RB - 1) / RB * ncomp;
-    const int grid = resident_grid(k_zreal<T, HH, RB, NTZ, C2R>, NTZ, zreal_smem<T, HH>(), work, cache);
-    k_zreal<T, HH, RB, NTZ, C2R><<<grid, NTZ, zreal_smem<T, HH>(), st>>>(a, ncomp);
-    return cudaGetLastError();
+    if constexpr (zreal_cta<T, HH>()) {
+      if (a.Mzp > z_row_cap<HH>()) return cudaErrorInvalidValue;
+      static PerDevice cache;
+      const long long work = (a.nrows + RB - 1) / RB * ncomp;
+      const int grid = resident_grid(k_zreal<T, HH, RB, NTZ, true>, NTZ, zreal_smem<T, HH>(), work, cache);
+      k_zreal<T, HH, RB, NTZ, true><<<grid, NTZ, zreal_smem<T, HH>(), st>>>(a, ncomp);
+      return cudaGetLastError();
+    } else {
+      return cudaErrorInvalidValue;
+    }
   });
 }
-template <typename T> cudaError_t launch_zc2r(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st) {
-  return launch_zreal<T, true>(H, a, ncomp, st);
-}
 template <typename T> cudaError_t launch_zr2c(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (zrealw_length(H)) return zrealw_ok(H, a) ? launch_zr2cw(H, a, ncomp, st) : cudaErrorInvalidValue;
+  }
   return dispatch_half(H, [&](auto hh) {
     constexpr int HH = decltype(hh)::value;
-    constexpr int RB = z_rows_per_block<HH>();
-    dim3 grid((a.nrows + RB - 1) / RB, ncomp);
-    k_zr2c<T, HH, RB, z_threads<HH>()><<<grid, z_threads<HH>(), zr2c_smem<T, HH>(), st>>>(a);
-    return cudaGetLastError();
+    if constexpr (zreal_cta<T, HH>()) {
+      constexpr int RB = z_rows_per_block<HH>();
+      dim3 grid((a.nrows + RB - 1) / RB, ncomp);
+      k_zr2c<T, HH, RB, z_threads<HH>()><<<grid, z_threads<HH>(), zr2c_smem<T, HH>(), st>>>(a);
+      return cudaGetLastError();
+    } else {
+      return cudaErrorInvalidValue;
+    }
   });
 }
 
@@ -961,9 +975,13 @@ template <typename T> cudaError_t prepare_fft_kernels(int Nx, int Ny, int Nz) {
     constexpr int HH = decltype(hh)::value;
     constexpr int RB = z_rows_per_block<HH>();
     constexpr int NTZ = z_threads<HH>();
-    cudaError_t r = max_smem(k_zreal<T, HH, RB, NTZ, true>, (int)zreal_smem<T, HH>());
-    if (r != cudaSuccess) return r;
-    return max_smem(k_zr2c<T, HH, RB, NTZ>, (int)zr2c_smem<T, HH>());
+    if constexpr (zreal_cta<T, HH>()) {
+      cudaError_t r = max_smem(k_zreal<T, HH, RB, NTZ, true>, (int)zreal_smem<T, HH>());
+      if (r != cudaSuccess) return r;
+      return max_smem(k_zr2c<T, HH, RB, NTZ>, (int)zr2c_smem<T, HH>());
+    } else {
+      return cudaSuccess;
+    }
   });
 }
 

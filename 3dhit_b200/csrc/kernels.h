@@ -215,12 +215,30 @@ template <typename K> int resident_grid(K kernel, int threads, size_t smem, long
 template <typename T> cudaError_t launch_axis(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, int nc, cudaStream_t st);
 template <typename T> cudaError_t launch_p1(const P1Args<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_p3(const P3Args<T>& a, cudaStream_t st);
+// Short columns (k_col.cu).  staged: the tiles can be staged by TMA / cp.async
+// (aligned rows); bytes: the pass's full side.  Both sides measured on the y
+// passes of 128^3 .. 512 x 128 x 256 grids: to 64 points k_col is faster or
+// equal everywhere; float64 at 128 too (33 against 39 us forward); float32 at
+// 128 only forward and within L2 (128^3 12.7 against 14.8 us; 512 x 128 x 256,
+// 138 MB, 69 against 64); with unaligned rows, which k_axis would read tile by
+// tile without staging, also at 256 (129 against 138).
+template <typename T> bool col_pass(int N, bool inv, bool staged, long long bytes) {
+  if (N <= 64 || (N == 128 && sizeof(T) == 8)) return true;
+  if (N == 128 && !inv && bytes <= (100LL << 20)) return true;
+  return N <= 256 && !staged;
+}
+template <typename T> cudaError_t launch_col(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, int nc, cudaStream_t st);
 // columns with xf_columns (k_xfield.cu)
 template <typename T> cudaError_t launch_p1f(const P1Args<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_p3f(const P3Args<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_zcross(int H, const ZCrossArgs<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_zc2r(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st);
 template <typename T> cudaError_t launch_zr2c(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st);
+// warp-resident forms (k_zrealw.cu): float32 rows of 64 .. 512 points
+constexpr bool zrealw_length(int H) { return H >= 32 && H <= 256; }
+bool zrealw_ok(int H, const ZRealArgs<float>& a);
+cudaError_t launch_zc2rw(int H, const ZRealArgs<float>& a, int ncomp, cudaStream_t st);
+cudaError_t launch_zr2cw(int H, const ZRealArgs<float>& a, int ncomp, cudaStream_t st);
 template <typename T> cudaError_t prepare_fft_kernels(int Nx, int Ny, int Nz);
 template <typename T> cudaError_t prepare_axis_kernels(int Nx);
 int p3_num_blocks(const Geom& g, int W);
