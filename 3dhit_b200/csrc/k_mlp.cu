@@ -247,8 +247,9 @@ __global__ void __launch_bounds__(128, 2) k_mlp_train(MlpArgs a) {
           dz[i] = 2.f * r * a.inv_count;
         }
       }
+      // (of the bf16 values that the weight gradients contract, as for the other biases)
 #pragma unroll
-      for (int i = 0; i < 6; ++i) db4[i] += dz[i];
+      for (int i = 0; i < 6; ++i) db4[i] += (double)__bfloat162float(__float2bfloat16_rn(dz[i]));
       store_row<16>(S.dz4, tid, dz, 16);
     }
     // ---- backward, two halves of 32 columns per layer ----
