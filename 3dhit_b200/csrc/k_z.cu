@@ -806,8 +806,10 @@ template <int HH, bool DA> cudaError_t launch_zwarp_v(const ZCrossArgs<float>& a
 }
 
 template <int HH> cudaError_t launch_zwarp(const ZCrossArgs<float>& a, cudaStream_t st) {
-  const bool da = a.Mz == zw_da_mz<HH>() && a.Mzp == (zw_da_mz<HH>() + 7) / 8 * 8;
-  return da ? launch_zwarp_v<HH, true>(a, st) : launch_zwarp_v<HH, false>(a, st);
+  if constexpr (HH <= 64) {  // longer rows of the dealiased layout: k_zw16
+    if (a.Mz == zw_da_mz<HH>() && a.Mzp == (zw_da_mz<HH>() + 7) / 8 * 8) return launch_zwarp_v<HH, true>(a, st);
+  }
+  return launch_zwarp_v<HH, false>(a, st);
 }
 
 template <bool DA> cudaError_t launch_zpair_v(const ZCrossArgs<float>& a, cudaStream_t st) {
@@ -833,8 +835,9 @@ cudaError_t launch_zpair(const ZCrossArgs<float>& a, cudaStream_t st) {
 }
 
 // float32 rows of Nz = 64 ... 1024 (whole row groups, staging rows of at most
-// H + 8 entries) take the warp-resident kernels (a warp pair per row at Nz =
-// 1024); every other case k_zcross.
+// H + 8 entries) take the warp-resident kernels: k_zw16 at Nz = 256 and 512 on
+// the dealiased layout, a warp pair per row at Nz = 1024, else k_zwarp; every
+// other case k_zcross.
 template <typename T> bool use_zwarp(int H, const ZCrossArgs<T>& a) {
   if (!std::is_same<T, float>::value || !(H == 32 || H == 64 || H == 128 || H == 256 || H == 512)) return false;
   const int rows = H <= 256 ? 256 / H : 1;
@@ -843,6 +846,7 @@ template <typename T> bool use_zwarp(int H, const ZCrossArgs<T>& a) {
 
 template <typename T> cudaError_t launch_zcross(int H, const ZCrossArgs<T>& a, cudaStream_t st) {
   if constexpr (std::is_same<T, float>::value) {
+    if (zw16_ok(H, a)) return launch_zw16(H, a, st);
     if (use_zwarp(H, a)) {
       if (H == 32) return launch_zwarp<32>(a, st);
       if (H == 64) return launch_zwarp<64>(a, st);

@@ -232,6 +232,8 @@ template <typename T> cudaError_t launch_col(int N, bool inv, const AxisArgs<T>&
 template <typename T> cudaError_t launch_p1f(const P1Args<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_p3f(const P3Args<T>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_zcross(int H, const ZCrossArgs<T>& a, cudaStream_t st);
+bool zw16_ok(int H, const ZCrossArgs<float>& a);  // k_zw16.cu
+cudaError_t launch_zw16(int H, const ZCrossArgs<float>& a, cudaStream_t st);
 template <typename T> cudaError_t launch_zc2r(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st);
 template <typename T> cudaError_t launch_zr2c(int H, const ZRealArgs<T>& a, int ncomp, cudaStream_t st);
 // warp-resident forms (k_zrealw.cu): float32 rows of 64 .. 512 points
@@ -249,6 +251,8 @@ cudaError_t set_axis_wait_limit(int polls);
 cudaError_t set_z_wait_limit(int polls);
 cudaError_t take_zadj_timeout(int* flag);
 cudaError_t take_plane_timeout(int* flag);
+cudaError_t take_zw16_timeout(int* flag);
+cudaError_t set_zw16_wait_limit(int polls);
 cudaError_t set_plane_wait_limit(int polls);
 cudaError_t set_zadj_wait_limit(int polls);
 template <typename T> int axis_tile_w(int N);

@@ -1757,11 +1757,12 @@ int hit_device_status(int* status) {
   int z = 0;
   cudaError_t e = take_axis_timeout(status);
   if (e == cudaSuccess) e = take_z_timeout(&z);
-  int za = 0, zp = 0;
+  int za = 0, zp = 0, zw = 0;
   if (e == cudaSuccess) e = take_zadj_timeout(&za);
   if (e == cudaSuccess) e = take_plane_timeout(&zp);
+  if (e == cudaSuccess) e = take_zw16_timeout(&zw);
   if (e != cudaSuccess) return cuda_fail(e, "device_status");
-  *status = *status || z || za || zp;
+  *status = *status || z || za || zp || zw;
   return HIT_OK;
 }
 
@@ -1770,6 +1771,7 @@ int hit_set_wait_limit(int polls) {
   if (e == cudaSuccess) e = set_z_wait_limit(polls);
   if (e == cudaSuccess) e = set_zadj_wait_limit(polls);
   if (e == cudaSuccess) e = set_plane_wait_limit(polls);
+  if (e == cudaSuccess) e = set_zw16_wait_limit(polls);
   return e == cudaSuccess ? HIT_OK : cuda_fail(e, "set_wait_limit");
 }
 
