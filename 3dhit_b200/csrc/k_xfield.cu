@@ -21,11 +21,15 @@
 // latencies overlap, and the layout's row bounds and 32-bit offsets fold most
 // of the address arithmetic into constants (a quarter of the instructions).
 // Time per launch of k_p3 -> k_p3f, stages with the fused x-inverse:
-//   256^3 float32, hold-energy sums  309 -> 203 us (586 MB: 0.44 of HBM)
-//   256^3 general layout             753 -> 637
-//   128 x 64 x 256                    60 -> 33
-//   64^3 general layout             40.5 -> 20.9
-//   128^3 float64                    102 -> 73
+//   256^3 float32, hold-energy sums  309 -> 168 us (586 MB: 0.53 of HBM)
+//   256^3 general layout             753 -> 547
+//   128 x 64 x 256                    60 -> 29
+//   64^3 hold-energy sums             31 -> 11
+//   128^3 float64                    102 -> 56
+// What bounds it now: the latency of a tile's two phases at two CTAs per SM.  A
+// one-group form for columns of 256 points (16 values per thread, the spectral
+// values in tensor memory, four CTAs per SM) measured 180 us and 20% more at
+// few tiles.
 #include "xfield.cuh"
 
 namespace hit {
@@ -71,7 +75,7 @@ __global__ void __launch_bounds__(XF_GROUPS* G, MINB) k_p3f(P3Args<T> a, int nzt
         const V2<T>* arr = q < 3 ? (a.stage <= 1 ? a.u : a.s) : (q < 6 ? a.acc : a.u);
         const V2<T>* base = arr + (q % 3) * a.c_c + cbase;
         for (int i = threadIdx.x - 3 * G; i < rows.Mx(); i += 2 * G)
-          prefetch_l2(base + (long long)i * a.c_x, W * sizeof(V2<T>));
+          prefetch_l2(base + (long long)i * a.c_x);
       }
       cta_sync();
     }
