@@ -167,6 +167,42 @@ template <bool INV, typename V> struct DFT<16, INV, V> {
   }
 };
 
+template <bool INV, typename V> struct DFT<32, INV, V> {
+  // n = 2 m + q: a DFT16 over m for each q, the odd one times W32^k, DFT2 over q.
+  static __device__ __forceinline__ void run(V* v) {
+    using T = decltype(v[0].x);
+    // cos and sin of pi k / 16
+    const T C[16] = {T(1), T(0.98078528040323044912618223613423904), T(0.92387953251128675612818318939678829),
+                     T(0.83146961230254523707878837761790575), T(0.70710678118654752440084436210484904),
+                     T(0.55557023301960222474283081394853287), T(0.38268343236508977172845998403039887),
+                     T(0.19509032201612826784828486847702224), T(0), T(-0.19509032201612826784828486847702224),
+                     T(-0.38268343236508977172845998403039887), T(-0.55557023301960222474283081394853287),
+                     T(-0.70710678118654752440084436210484904), T(-0.83146961230254523707878837761790575),
+                     T(-0.92387953251128675612818318939678829), T(-0.98078528040323044912618223613423904)};
+    V e[16], o[16];
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+      e[m] = v[2 * m];
+      o[m] = v[2 * m + 1];
+    }
+    DFT<16, INV, V>::run(e);
+    DFT<16, INV, V>::run(o);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      V t;
+      if (k == 0) t = o[0];
+      else if (k == 8) t = INV ? cmul_i(o[8]) : cmul_mi(o[8]);
+      else {
+        const T c = C[k], s = (INV ? T(1) : T(-1)) * C[k <= 8 ? 8 - k : k - 8];  // sin(pi k/16) = cos(pi (8 - k)/16)
+        t.x = o[k].x * c - o[k].y * s;
+        t.y = o[k].y * c + o[k].x * s;
+      }
+      v[k] = cadd(e[k], t);
+      v[k + 16] = csub(e[k], t);
+    }
+  }
+};
+
 struct NoHook {
   __device__ void operator()() const {}
 };

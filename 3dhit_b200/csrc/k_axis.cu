@@ -24,6 +24,7 @@
 #include "p3_epilogue.cuh"
 #include "tc_common.cuh"
 #include "tma.cuh"
+#include "xfield.cuh"
 
 namespace hit {
 
@@ -161,6 +162,117 @@ __global__ void __launch_bounds__(NT) k_axis(AxisArgs<T> a, int nzt, int no, int
     walk = nwalk;
   }
   if constexpr (PF == 1) cp_async_wait_all();
+}
+
+// k_axis with TMA staging for columns whose transform fits two stages in
+// registers (Two<N>: 128, 256 and, in float32, 512 points as 16 x 32): a value
+// crosses shared memory three times as an LSU operand (staged tile, exchange
+// out and in) instead of five.  k_axis is bound by that path (72 to 75% of its
+// wavefronts in ncu).  16 values per thread (32 at 512 points), two barriers per
+// tile; the next tile's boxes are requested when all threads hold the staged
+// values.
+template <typename T, int N> struct Axis2 {
+  static constexpr int W = tile_w<T>(N);
+  static constexpr int G = N * W / (N == 512 ? 32 : 16);
+    static constexpr int MINB = N == 512 ? 2 : (sizeof(T) == 8 ? 4 : 640 / G);
+  using XT = XTile<N, W>;
+  // exchange tile, twiddles, staged tile on a 128-byte boundary
+  static constexpr size_t smem = sizeof(V2<T>) * (size_t)(XT::SLOTS + XT::TWS + N * W) + 128;
+};
+// Both sides measured per pass, k_axis -> k_axis2: the 2/3 box 95 -> 82 us (256^3
+// inverse; forward 49.5 -> 41.8), 717 -> 644 (512^3), 17.7 -> 16.8 (128^3); all rows
+// stored, 26.9 -> 23.6 (57 MB, 64 x 256 x 128), forward 44.7 -> 43.1 (113 MB), but
+// 80.6 -> 90.9 at 226 MB and 1137 -> 1660 at 512^3, where the passes are beyond L2
+// and k_axis's fewer, larger CTAs keep more of the traffic in order; at 128 points
+// the line lies higher (86 against 94 at 214 MB, 169 against 190 at 415 MB, 375
+// against 346 at 830 MB).
+template <typename T> bool axis2_pass(int N, bool box, long long bytes) {
+  return box || bytes <= ((N == 128 ? 512LL : 128LL) << 20);
+}
+template <typename T> constexpr bool axis_two(int N) { return sizeof(T) == 4 ? N >= 128 && N <= 512 : N == 256; }
+
+// ROWS: 1 the compact side is the 2/3 box, 0 any
+template <typename T, int N, bool INV, int ROWS>
+__global__ void __launch_bounds__(Axis2<T, N>::G, Axis2<T, N>::MINB)
+    k_axis2(AxisArgs<T> a, int nzt, int no, int ntiles, const __grid_constant__ CUtensorMap mapA,
+            const __grid_constant__ CUtensorMap mapB) {
+  constexpr int W = Axis2<T, N>::W, G = Axis2<T, N>::G;
+  constexpr bool EARLY = N == 512 && INV;  // ask for the next tile before the first stage, not after
+  using XT = XTile<N, W>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t tbar;
+  V2<T>* tws = reinterpret_cast<V2<T>*>(smem_raw);
+  V2<T>* x = tws + XT::TWS;
+  V2<T>* stg = reinterpret_cast<V2<T>*>((reinterpret_cast<uintptr_t>(x + XT::SLOTS) + 127) & ~(uintptr_t)127);
+  constexpr int XE = sizeof(V2<T>) / 8;  // 8-byte tensor elements per complex value
+  const int tl = threadIdx.x;
+  const uint32_t mb = tma::smem_u32(&tbar);
+  xf_twiddles<T, N, W>(tws, a.tw);
+  const ColRows<N, ROWS == 1> rows{INV ? a.hin : a.hout, INV ? a.Min : a.Mout};
+  auto request = [&](const TileWalk& w) {
+    if (tl == 0) {
+      tma::mbar_expect_tx(mb, (uint32_t)((a.ka + a.kb) * a.br * W * sizeof(V2<T>)));
+      const int xc = w.zt * W * XE;
+      for (int k = 0; k < a.ka; ++k) tma::load4(stg + k * a.br * W, &mapA, xc, k * a.br, w.o, w.c, mb);
+      for (int k = 0; k < a.kb; ++k)
+        tma::load4(stg + (N - (k + 1) * a.br) * W, &mapB, xc, a.pb - (k + 1) * a.br, w.o, w.c, mb);
+    }
+  };
+  for (int e = tl; e < (N - (a.ka + a.kb) * a.br) * W; e += G) stg[a.ka * a.br * W + e] = czero<T>();
+  if (tl == 0) tma::mbar_init(mb, 1);
+  tma::fence_async_smem();
+  TileWalk walk(blockIdx.x, gridDim.x, nzt, no);
+  const int wait_limit = g_axis_wait_limit;
+  pdl_wait();
+  __syncthreads();
+  if (blockIdx.x < ntiles) request(walk);
+  constexpr uint32_t ES = sizeof(V2<T>);
+  const uint32_t da = (uint32_t)a.d_a * ES;
+  uint32_t phase = 0;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int z0 = walk.zt * W;
+    V2<T>* dst = a.dst + walk.c * a.d_c + walk.o * a.d_o + z0;
+    const int nc = a.nz - z0;  // valid columns of the tile
+    // the tile's boxes have landed (a verdict shared by the block, whose
+    // threads have also left the exchange tile)
+    const bool ok = __syncthreads_and(tma::mbar_wait(mb, phase, wait_limit)) != 0;
+    phase ^= 1;
+    if (!ok) {
+      if (tl == 0) atomicExch(&g_axis_timeout, 1);
+      tma::mbar_wait(mb, phase ^ 1, AXIS_WAIT);  // the copies in flight, once more with a limit
+      return;
+    }
+    const TileWalk nwalk = walk.next();
+    Stage0<T, N, W, G> s0;
+    s0.load(tl, [&](int b, int lo, int col) {
+      if (INV && ROWS == 1 && rows.row(0, lo, XT::R1) < 0 && rows.row(XT::R1 - 1, lo, XT::R1) < 0) return czero<T>();
+      return stg[(lo + b) * W + col];
+    });
+    if (EARLY) {
+      __syncthreads();
+      if (tile + (int)gridDim.x < ntiles) request(nwalk);
+    }
+    s0.template store<INV>(tl, x);
+    __syncthreads();
+    if (!EARLY && tile + (int)gridDim.x < ntiles) request(nwalk);
+    xf_stage1<T, N, W, G, INV>(tl, x, tws, [&](int b, int lo, int col, V2<T> v, V2<T>*) {
+      const int row = INV ? lo + b : rows.row(b, lo, XT::R0);
+      if (row >= 0 && col < nc) elem(dst, (uint32_t)row * da + (uint32_t)col * ES) = v;
+    });
+    walk = nwalk;
+  }
+}
+
+template <typename T, int N, bool INV, int ROWS>
+cudaError_t launch_axis2(const AxisArgs<T>& a, int nzt, int no, long long ntiles, const CUtensorMap& mA,
+                         const CUtensorMap& mB, cudaStream_t st) {
+  using C = Axis2<T, N>;
+  constexpr auto kernel = k_axis2<T, N, INV, ROWS>;
+  static PerDevice ready, cache;
+  cudaError_t e = once_per_device(ready, [] { return xf_attr(kernel, C::smem); });
+  if (e != cudaSuccess) return e;
+  return launch_pdl(kernel, resident_grid(kernel, C::G, C::smem, ntiles, cache), C::G, C::smem, st, a, nzt, no,
+                    (int)ntiles, mA, mB);
 }
 
 // x-inverse of u and w = i k x u for one (ky row, z tile).  comp(c, pos, col,
@@ -1023,6 +1135,18 @@ cudaError_t launch_axis(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, 
                        axis_map<T>(&mB, a.src + (long long)a.hin * a.s_a, cols, t.pb, no, nc, a.s_a, a.s_o, a.s_c, W,
                                    t.br);
       const size_t smem = axis_smem<T, NN, W, true>();
+      if constexpr (axis_two<T>(NN)) {
+        const int M = inv ? a.Min : a.Mout, h = inv ? a.hin : a.hout;
+        const bool box = M == 2 * (NN / 3) + 1 && h == NN / 3 + 1;
+        if (tma && axis2_pass<T>(NN, box, ntiles * NN * W * (long long)sizeof(V2<T>)) &&
+            (unsigned long long)a.d_a * NN * sizeof(V2<T>) < (1ULL << 32)) {  // 32-bit byte offsets along the axis
+          if (inv)
+            return box ? launch_axis2<T, NN, true, 1>(t, nzt, no, ntiles, mA, mB, st)
+                       : launch_axis2<T, NN, true, 0>(t, nzt, no, ntiles, mA, mB, st);
+          return box ? launch_axis2<T, NN, false, 1>(t, nzt, no, ntiles, mA, mB, st)
+                     : launch_axis2<T, NN, false, 0>(t, nzt, no, ntiles, mA, mB, st);
+        }
+      }
       if (tma) {
         if (inv)
           return launch_pdl(k_axis<T, NN, W, true, 2>, resident_grid(k_axis<T, NN, W, true, 2>, NT, smem, ntiles, c[4]),

@@ -12,29 +12,12 @@
 // k_axis works on one tile per CTA, whose 256 threads have no butterfly at all
 // in most short stages.  Six y-inverse fields, k_axis -> k_col: 512 x 16 x 512
 // 86 -> 27 us, 512 x 32 x 512 107 -> 58, 512 x 64 x 512 125 -> 107, 64 points in
-// 128 x 64 x 256 19 -> 15.  At 128 and 256 points k_axis's tiles fill its
-// threads, and its TMA staging sustains 4.8 TB/s against 3.6 here (256^3: 95
-// against 124 us), whatever the number of loads in flight (next tile's loads
-// held in registers: 127).
+// 128 x 64 x 256 19 -> 15.  At 128 and 256 points TMA staging (k_axis2) is
+// faster (256^3: 82 against 124 us), whatever the number of loads in flight here
+// (next tile's loads held in registers: 127).
 #include "xfield.cuh"
 
 namespace hit {
-
-// Stored rows of one side: compile-time when they are the 2/3 box (DA).
-template <int N, bool DA> struct ColRows {
-  int h_, M_;
-  __device__ __forceinline__ int h() const { return DA ? N / 3 + 1 : h_; }
-  __device__ __forceinline__ int M() const { return DA ? 2 * (N / 3) + 1 : M_; }
-  // stored row of position lo + b, b in [0, nb) (nb and lo constants), or -1
-  __device__ __forceinline__ int row(int b, int lo, int nb) const {
-    const int off = N - M();
-    if (DA && lo + nb <= h()) return lo + b;
-    if (DA && lo >= h() + off) return lo + b - off;
-    if (DA && lo >= h() && lo + nb <= h() + off) return -1;
-    const int pos = lo + b;
-    return pos < h() ? pos : (pos >= h() + off ? pos - off : -1);
-  }
-};
 
 constexpr int COL_THREADS = 256;
 template <typename T, int N> struct ColCfg {

@@ -14,8 +14,8 @@ namespace hit {
 // Radices of the two stages.
 template <int N> struct Two {
   static constexpr int L = ilog2(N);
-  static constexpr int R0 = 1 << (L / 2), R1 = N / R0;  // R0 <= R1 <= 16
-  static_assert(N >= 4 && R1 <= 16, "two-stage columns");
+  static constexpr int R0 = 1 << (L / 2), R1 = N / R0;  // R0 <= R1 <= 32
+  static_assert(N >= 4 && R1 <= 32, "two-stage columns");
 };
 
 // Shared-memory layout of a field's exchange tile: slot (pos + pos / R0) W +
@@ -46,6 +46,22 @@ __device__ __forceinline__ void xf_twiddles(V2<T>* tws, const V2<T>* __restrict_
   for (int e = threadIdx.x; e < (X::R1 - 1) * X::R0; e += blockDim.x)
     tws[e] = tw[(e / X::R0 + 1) * (e % X::R0) * (TWN / N)];
 }
+
+// Stored rows of one side: compile-time when they are the 2/3 box (DA).
+template <int N, bool DA> struct ColRows {
+  int h_, M_;
+  __device__ __forceinline__ int h() const { return DA ? N / 3 + 1 : h_; }
+  __device__ __forceinline__ int M() const { return DA ? 2 * (N / 3) + 1 : M_; }
+  // stored row of position lo + b, b in [0, nb) (nb and lo constants), or -1
+  __device__ __forceinline__ int row(int b, int lo, int nb) const {
+    const int off = N - M();
+    if (DA && lo + nb <= h()) return lo + b;
+    if (DA && lo >= h() + off) return lo + b - off;
+    if (DA && lo >= h() && lo + nb <= h() + off) return -1;
+    const int pos = lo + b;
+    return pos < h() ? pos : (pos >= h() + off ? pos - off : -1);
+  }
+};
 
 // The stored x rows: compile-time for the dealiased layout (DA), so that the
 // bounds of a butterfly's positions fold into constants.
