@@ -108,7 +108,11 @@ template <typename T> struct KTab {
 // while the previous kernel in the stream is still finishing.  It sets up what
 // depends on no earlier kernel (twiddle tables, shared-memory zero fill), then
 // pdl_wait() returns once the previous grid has completed and its writes are
-// visible; pdl_trigger() then lets the next kernel start launching.
+// visible; pdl_trigger() then lets the next kernel start launching.  A kernel
+// without it lets the next one start as its own blocks end, which is faster where
+// early blocks of the next kernel would take up unevenly what this one leaves free
+// (k_axis and k_axis2: 128 x 256 x 128 float64 step 1288 us with it, 1068 without;
+// to_physical and to_spectral of 256^3 610 us, 519 without).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 

@@ -118,7 +118,6 @@ __global__ void __launch_bounds__(NT) k_axis(AxisArgs<T> a, int nzt, int no, int
   TileWalk walk(blockIdx.x, gridDim.x, nzt, no);
   const int wait_limit = PF == 2 ? g_axis_wait_limit : 0;
   pdl_wait();
-  pdl_trigger();
   __syncthreads();
   if (PF != 0 && blockIdx.x < ntiles) prefetch(walk);
   if constexpr (PF != 2) __syncthreads();

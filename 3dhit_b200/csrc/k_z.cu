@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(NWARP * 32, ZW_MINB) k_zwarp(ZCrossArgs<float>
   };
 
   pdl_wait();
-  pdl_trigger();
+  if (DA) pdl_trigger();  // (general layout: step of 512 x 256 x 128 3250 us with it, 3113 without)
   long long grp = (long long)blockIdx.x * NWARP + warp;
   if (grp < ngroups) prefetch(grp);
   uint32_t phase = 0;
