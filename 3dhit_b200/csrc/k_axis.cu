@@ -9,7 +9,8 @@
 // straight to global memory (or to the fused epilogue); only the middle stages
 // go through shared memory.
 //
-// k_p1 and k_p3 are the x-axis ends of the RHS (src/hit3d/navierstokes.py:69-95):
+// k_p1 and k_p3 (k_p3m at 512 float32 points) are the x-axis ends of the RHS
+// (src/hit3d/navierstokes.py:69-95) for the columns that k_xfield.cu does not serve:
 //   k_p1: curl (navierstokes.py:73-77) and the x part of to_physical for u and w;
 //   k_p3: x part of to_spectral, forcing (forcing.py:94-95,138-143), dealias +
 //         projection (grid.py:166-178), viscous term (navierstokes.py:95) and

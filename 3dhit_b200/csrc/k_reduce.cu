@@ -389,13 +389,6 @@ struct Kahan {
   }
 };
 
-// Deterministic block-wide Kahan sum of column v of partial[nb][stride].
-__device__ double kahan_column(const double* partial, int nb, int stride, int v, double* red) {
-  Kahan k;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) k.add(partial[(long long)b * stride + v]);
-  return block_sum_f64(k.s - k.c, red);
-}
-
 __device__ __forceinline__ double forcing_coef(int forcing, double E, double Om, double twoEb, double nu, double eps,
                                                double Et, double tau, double tiny, double A) {
   if (forcing == 1) return A;

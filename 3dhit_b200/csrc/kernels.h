@@ -43,9 +43,8 @@ template <typename T> __host__ __device__ constexpr int tile_wp(int N) { return 
 
 // Column lengths of the field-parallel x kernels (k_xfield.cu) and their tile
 // width.  Longer columns do not fit five exchange tiles per CTA with two CTAs
-// on an SM; float64 columns of 256 points just do on the dealiased layout (433
-// us against k_p3's 428 per launch at 256^3) and not on the general one (1578
-// against 1100), so they stay with k_p3.
+// on an SM; float64 columns of 256 points do on the dealiased layout only (371
+// us against k_p3's 387 per launch at 256^3), so they stay with k_p3.
 template <typename T> __host__ __device__ constexpr bool xf_columns(int N) { return N <= (sizeof(T) == 4 ? 256 : 128); }
 template <typename T> __host__ __device__ constexpr int xf_tile_w() { return 64 / (int)sizeof(V2<T>); }
 

@@ -8,9 +8,10 @@
 //                 the y/z-forward products (T3)
 //   U6            x,y-physical u and w (6 comps); first 3 comps: z-forward u x w
 // One RHS evaluation (src/hit3d/navierstokes.py:69-95) is
-//   P1 (x-inverse, k_p1)  -> P2a (y-inverse)  -> P2b (z c2r, u x w, z r2c)
-//   -> P2c (y-forward)    -> P3 (x-forward + forcing/dealias/projection/
+//   P1 (x-inverse)      -> P2a (y-inverse)  -> P2b (z c2r, u x w, z r2c)
+//   -> P2c (y-forward)  -> P3 (x-forward + forcing/dealias/projection/
 //                              viscous/RK update + next stage's P1)
+// (P2a to P2c in one kernel on small planes, k_plane.cu)
 // and one RK4 step (src/hit3d/integrators.py:32-38) is four such chains.  A
 // rollout (integrators.py:41-53, the replacement for lax.scan) runs P1 once,
 // then replays a captured CUDA graph of one step whose last P3 also prepares

@@ -165,14 +165,15 @@ int hit_rollout(hit_plan *plan, const void *u_hat, const hit_params *params,
  * custom_vjp rule conjugates them on the way in and out).  param_ct_dev, when
  * not NULL, is a DEVICE double[3] that receives the cotangents of (nu, A, eps)
  * of `params` (A: linear forcing; eps: band forcing; for the hold-energy
- * forcing nu also enters its coefficient).  The transposes run on the general
- * (full-layout) path in the plan's dtype and recompute what they need:
+ * forcing nu also enters its coefficient).  The transposes run in the plan's
+ * dtype (on the 2/3 box inside when params carries HIT_FLAG_ASSUME_DEALIASED,
+ * which states that u_hat lies in it; ct may be any) and recompute what they need:
  *   hit_rhs_vjp       u_bar = (d rhs/d u)^T ct at u_hat;
  *   hit_rk4_step_vjp  u_bar = (d rk4_step/d u)^T ct (stage inputs recomputed);
  *   hit_rollout_vjp   u0_bar = (d rollout/d u0)^T ct: states are kept every
  *                     checkpoint_every steps, each segment is recomputed and
  *                     transposed step by step (memory: nsteps/checkpoint_every
- *                     + checkpoint_every states).
+ *                     states and those of one segment).
  * u_bar may alias ct. */
 int hit_rhs_vjp(hit_plan *plan, const void *u_hat, const hit_params *params,
                 double t, const void *ct, void *u_bar, double *param_ct_dev,
@@ -313,7 +314,7 @@ int hit_axis_fft(hit_plan *plan, const void *in, void *out, int ncomp,
  * the RK4 step with the force f_ext held over its stages: u_bar = (d step /
  * d u)^T ct, f_bar (nullable) = (d step / d f_ext)^T ct = P (sum of the
  * stages' cotangents), P the dealias mask and projection; param_ct as in
- * hit_rk4_step_vjp.  The stage inputs are recomputed on the general path. */
+ * hit_rk4_step_vjp.  The stage inputs are recomputed. */
 int hit_rk4_step_forced_vjp(hit_plan *plan, const void *u_hat,
                             const hit_params *params, const void *f_ext,
                             double dt, double t, const void *ct, void *u_bar,
