@@ -23,7 +23,7 @@
 // Time per launch of k_p3 -> k_p3f, stages with the fused x-inverse:
 //   256^3 float32, hold-energy sums  309 -> 168 us (586 MB: 0.53 of HBM)
 //   256^3 general layout             753 -> 547
-//   128 x 64 x 256                    60 -> 29
+//   128 x 64 x 256                    60 -> 27
 //   64^3 hold-energy sums             31 -> 11
 //   128^3 float64                    102 -> 56
 // What bounds it now: the latency of a tile's two phases at two CTAs per SM.  A

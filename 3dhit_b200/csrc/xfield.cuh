@@ -208,7 +208,10 @@ __device__ __forceinline__ void xf_inverse(const V2<T>* F, V2<T>* X, const V2<T>
 // ---------------------------------------------------------------------------
 
 // Tile width (64-byte row segments), threads per group and CTAs per SM that
-// the register budget is sized for.
+// the register budget is sized for.  x-forward pass at 128 float points, budget
+// for 2, 3 and 4 CTAs: general 128^3 66, 70 and 81 us, 2/3 box of 128 x 64 x 256
+// 27.4, 27.9 and 28.9; at 64 points 10.7, 10.7 (3) and 12.2 (4), general 18.6, 16.2,
+// 16.7; float64 57 us for 2 CTAs, 76 for 3, 63 for 1.
 template <typename T, int N, bool DA> struct XfCfg {
   static constexpr int W = xf_tile_w<T>();
   static constexpr int B = Two<N>::R1 * W;  // stage-0 butterflies of a transform
@@ -217,7 +220,7 @@ template <typename T, int N, bool DA> struct XfCfg {
   // exchange tiles, one CTA per SM
   static constexpr bool WIDE = N == 256 && !DA;
   static constexpr int G = B < 64 ? 32 : (WIDE ? B : 64);
-  static constexpr int MINB = WIDE ? 1 : (F32 ? (N == 256 ? 2 : (N == 128 ? 4 : 3)) : 2);
+  static constexpr int MINB = WIDE ? 1 : (F32 ? (N >= 128 ? 2 : 3) : 2);
 };
 
 // Slot offset of F from X: over the exchange tiles of groups 3 and 4 (idle
