@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(XA_GROUPS* G, MINB) k_adjx2(AdjX2Args<T> a, in
   const uint32_t rx = (uint32_t)g.Ny * (uint32_t)g.Mzp * ES, cx = (uint32_t)a.c_x * ES;
   const double* sc = a.scal;
   const T a_all = (T)sc[0], a_band = (T)sc[1], c_w = (T)sc[2], c_wk2 = (T)sc[3], c_wb = (T)sc[4];
+  T nf = T(0);  // sum of 0 v over the modes that the state does not store: NaN where v is not finite
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int j = tile / nzt, z0 = (tile % nzt) * W, z = z0 + col;
     const uint32_t tb = ((uint32_t)j * (uint32_t)g.Mzp + z0) * ES;
@@ -175,6 +176,7 @@ __global__ void __launch_bounds__(XA_GROUPS* G, MINB) k_adjx2(AdjX2Args<T> a, in
           if (a.mode >= 1 && a.mode <= 3) ac[c] = elem((const V2<T>*)a.acc + c * r_c, o);
           if (a.fb && !a.fb_first) fb[c] = elem((const V2<T>*)a.fb + c * r_c, o);
           pv[c] = v[c];
+          if (!in) nf += T(0) * v[c].x + T(0) * v[c].y;
         }
         Mode<T> d;
         d.kx = __ldg(a.k.kx + pos);
@@ -209,6 +211,9 @@ __global__ void __launch_bounds__(XA_GROUPS* G, MINB) k_adjx2(AdjX2Args<T> a, in
       }
     }
   }
+  // nu's cotangent is -sum k2 Re(conj(v) u) over all modes; k_adjx1 sums those of
+  // the box, the others add 0 v
+  if (nf != T(0)) atomicAdd(a.pct, (double)nf);
 }
 
 // One warp per sum: Kahan over the blocks' partials (lane stride 32), a fixed

@@ -353,6 +353,7 @@ template <typename T> struct AdjX2Args {
   const V2<T>* tw;
   T nu, kmin2, kmax2;
   const double* scal;
+  double* pct;       // parameter cotangents, [0] nu's
 };
 template <typename T> struct ZAdjArgs {
   const V2<T>* in;   // (9, Nx, Ny, Mzp): x, y-physical u, om, g

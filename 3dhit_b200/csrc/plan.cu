@@ -1284,6 +1284,7 @@ int adj_stage(hit_plan* p, Path& P, const Scalars& s, const AdjStage<T>& q, cons
   y.kmin2 = (T)s.kmin2;
   y.kmax2 = (T)s.kmax2;
   y.scal = static_cast<const double*>(p->ascal.p);
+  y.pct = pct;
   HIT_CK(launch_adj_x2<T>(y, st));
   return HIT_OK;
 }
