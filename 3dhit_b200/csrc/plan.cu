@@ -1668,6 +1668,7 @@ int hit_plan_destroy(hit_plan* p) {
     release(P.D);
     release(P.partial);
     release(P.coef);
+    release(P.FEXT);
   }
   release(p->ktab);
   release(p->tw);
