@@ -16,7 +16,8 @@ in include/hit3d.h):
 Cotangents are dL/dRe + i dL/dIm of the stored half-spectrum entries, which
 is PyTorch's convention for complex tensors (``jax.vjp`` returns the complex
 conjugate).  The rollout keeps a state every ``checkpoint_every`` steps and
-recomputes each segment, so memory is (nsteps / K + K) states.
+recomputes each segment, so memory is (nsteps / K + K) states, and eight more for
+the stage inputs of a state in the 2/3 box.
 """
 
 from __future__ import annotations

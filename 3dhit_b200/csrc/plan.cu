@@ -156,9 +156,9 @@ struct hit_plan {
   // cotangents, and the rollout checkpoints
   Buf ax9, aph, as6, apart, asums, ascal, apct, ast[3], ak, akb, asb, aacc, aub, ack, aseg, afb;
   // of the fused transpose (columns with xf_columns): x- and x,y-physical
-  // fields, products; cotangents in the padded general layout; stage inputs of
-  // one step, and of every step of a segment on the dealiased layout
-  Buf at9, au9, ar6, avb, avk, ava, avf, asg;
+  // fields, products; cotangents in the padded general layout; a segment's store
+  // on the dealiased layout and its states' forcing coefficients
+  Buf at9, au9, ar6, avb, avk, ava, avf, asg, acoef;
   cudaStream_t cap = nullptr;  // private stream used only for graph capture
   // side branch of the step for the forcing coefficient's reduction (see
   // fork_coef): its stream and one fork / join event pair per RK4 stage
@@ -188,6 +188,8 @@ template <typename T> V2<T>* vp(const Buf& b) { return static_cast<V2<T>*>(b.p);
 
 bool needs_coef(int forcing) { return forcing == HIT_FORCING_BAND || forcing == HIT_FORCING_HOLD_ENERGY; }
 
+constexpr size_t COEF_BYTES = 8 * sizeof(double);  // a path's forcing coefficient and its sums (CoefArgs)
+
 template <typename T> int ensure_path(hit_plan* p, int which) {
   Path& P = p->path[which];
   if (P.ready) return HIT_OK;
@@ -208,7 +210,7 @@ template <typename T> int ensure_path(hit_plan* p, int which) {
   P.gather_blocks = (int)std::min<long long>((nm + NT - 1) / NT, 8 * 148);
   const int nb = std::max(P.p3_blocks, P.gather_blocks);
   if ((rc = ensure(P.partial, (size_t)3 * nb * sizeof(double)))) return rc;
-  if ((rc = ensure(P.coef, 8 * sizeof(double)))) return rc;
+  if ((rc = ensure(P.coef, COEF_BYTES))) return rc;
   P.ready = true;
   return HIT_OK;
 }
@@ -1423,10 +1425,17 @@ int rk4_vjp_fused(hit_plan* p, const void* u, const hit_params* pr, double dt, c
 
 // u0_bar = (d rollout / d u0)^T ub: states every K steps are kept (reference
 // layout), each segment is run forwards again and transposed step by step.  On
-// the dealiased layout a compact state is a third of a full one, and the
-// segment keeps all four stage inputs of its steps, so nothing is recomputed
-// twice; on the general layout it keeps the steps' states and recomputes the
-// stage inputs.
+// the dealiased layout the segment keeps its steps' states in the compact layout
+// and, of its first `keep` steps, the three other stage inputs too; those of a
+// later step are formed again when its turn comes.  The store takes no more than
+// K + SEG_EXTRA full states: with the 15 (at 128^3 and above) of the rest of this
+// path's workspace the call stays below the 26 and K that the transposes in the
+// reference layout hold, for any K.  A compact state is 0.30 to 0.33 of a full
+// one on cubes from 64^3, so every stage input is kept up to K = 25 (64^3), 26
+// (128^3) or 36 (256^3).  Where padding makes the compact state the larger one
+// (rows of four points), and on the general layout, the segment keeps full
+// states and forms the stage inputs again.
+constexpr int SEG_EXTRA = 8;
 template <typename T>
 int rollout_vjp_fused(hit_plan* p, const void* u0, const hit_params* pr, double dt, int64_t nsteps, int K,
                       const void* ub, void* u0_bar, double* pct, cudaStream_t st) {
@@ -1445,8 +1454,15 @@ int rollout_vjp_fused(hit_plan* p, const void* u0, const hit_params* pr, double 
   const long long cmp = 3LL * P.g.Mx * P.g.My * P.g.Mzp;
   if ((rc = ensure(p->ack, nseg * bytes))) return rc;
   if ((rc = ensure(p->avb, cotangent_bytes<T>(p)))) return rc;
-  if (which) {
-    if ((rc = ensure(p->asg, (size_t)4 * K * cmp * sizeof(V2<T>)))) return rc;
+  const bool compact = which && cmp <= n;
+  const int keep = compact ? (int)std::min<long long>(K, ((K + SEG_EXTRA) * n - K * cmp) / (3 * cmp)) : 0;
+  const bool red = needs_coef(s.forcing);
+  if (compact) {
+    if ((rc = ensure(p->asg, (K + 3LL * keep) * cmp * sizeof(V2<T>)))) return rc;
+    if (keep < K)
+      for (Buf& b : p->ast)
+        if ((rc = ensure(b, cmp * sizeof(V2<T>)))) return rc;
+    if (red && (rc = ensure(p->acoef, K * COEF_BYTES))) return rc;
   } else {
     if ((rc = ensure(p->aseg, (size_t)K * bytes))) return rc;
   }
@@ -1458,17 +1474,36 @@ int rollout_vjp_fused(hit_plan* p, const void* u0, const hit_params* pr, double 
     if ((rc = rollout_impl<T>(p, CK + (j - 1) * n, pr, dt, K, CK + j * n, nullptr, st))) return rc;
   for (int64_t j = nseg - 1; j >= 0; --j) {
     const int len = (int)std::min<int64_t>(K, nsteps - j * K);
-    if (which) {
+    if (compact) {
       V2<T>* A = vp<T>(p->asg);
+      struct Inputs {
+        V2<T>* S[3];
+      };
+      auto inputs = [&](int i) {  // stage inputs 2..4 of step i
+        V2<T>* q = A + (K + 3LL * i) * cmp;
+        return i < keep ? Inputs{{q, q + cmp, q + 2 * cmp}} : Inputs{{vp<T>(p->ast[0]), vp<T>(p->ast[1]), vp<T>(p->ast[2])}};
+      };
+      // the forcing coefficient of a step's state, for the steps that run twice
+      auto coef_copy = [&](int i, bool save) -> int {
+        void* slot = static_cast<char*>(p->acoef.p) + i * COEF_BYTES;
+        HIT_CK(cudaMemcpyAsync(save ? slot : P.coef.p, save ? P.coef.p : slot, COEF_BYTES, cudaMemcpyDeviceToDevice, st));
+        return HIT_OK;
+      };
       if ((rc = gather_state<T>(p, P, CK + j * n, s, st, A))) return rc;
       for (int i = 0; i < len; ++i) {
-        V2<T>* u = A + 4LL * i * cmp;
-        V2<T>* S[3] = {u + cmp, u + 2 * cmp, u + 3 * cmp};
-        if ((rc = adj_forward<T>(p, P, s, dt, u, S, i + 1 < len ? u + 4 * cmp : nullptr, i > 0, nullptr, st))) return rc;
+        V2<T>* u = A + i * cmp;
+        if (red && i >= keep && (rc = coef_copy(i, true))) return rc;
+        if ((rc = adj_forward<T>(p, P, s, dt, u, inputs(i).S, i + 1 < len ? u + cmp : nullptr, i > 0, nullptr, st)))
+          return rc;
       }
       for (int i = len - 1; i >= 0; --i) {
-        const V2<T>* u = A + 4LL * i * cmp;
-        const V2<T>* states[4] = {u, u + cmp, u + 2 * cmp, u + 3 * cmp};
+        V2<T>* u = A + i * cmp;
+        const Inputs in = inputs(i);
+        if (i >= keep && i + 1 < len) {  // (the last step's are still there)
+          if (red && (rc = coef_copy(i, false))) return rc;
+          if ((rc = adj_forward<T>(p, P, s, dt, u, in.S, nullptr, false, nullptr, st))) return rc;
+        }
+        const V2<T>* states[4] = {u, in.S[0], in.S[1], in.S[2]};
         if ((rc = adj_step<T>(p, P, s, dt, states, VB, nullptr, pct, st))) return rc;
       }
     } else {
@@ -1677,7 +1712,8 @@ int hit_plan_destroy(hit_plan* p) {
   release(p->dsums);
   for (Buf* b : {&p->ax9, &p->aph, &p->as6, &p->apart, &p->asums, &p->ascal, &p->apct, &p->ast[0], &p->ast[1],
                  &p->ast[2], &p->ak, &p->akb, &p->asb, &p->aacc, &p->aub, &p->ack, &p->aseg, &p->afb, &p->at9,
-                 &p->au9, &p->ar6, &p->avb, &p->avk, &p->ava, &p->avf, &p->asg})
+                 &p->au9, &p->ar6, &p->avb, &p->avk, &p->ava, &p->avf, &p->asg,
+                 &p->acoef})
     release(*b);
   if (p->cap) cudaStreamDestroy(p->cap);
   if (p->side) cudaStreamDestroy(p->side);

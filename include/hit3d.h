@@ -173,7 +173,7 @@ int hit_rollout(hit_plan *plan, const void *u_hat, const hit_params *params,
  *   hit_rollout_vjp   u0_bar = (d rollout/d u0)^T ct: states are kept every
  *                     checkpoint_every steps, each segment is recomputed and
  *                     transposed step by step (memory: nsteps/checkpoint_every
- *                     states and those of one segment).
+ *                     + checkpoint_every + 8 states at most).
  * u_bar may alias ct. */
 int hit_rhs_vjp(hit_plan *plan, const void *u_hat, const hit_params *params,
                 double t, const void *ct, void *u_bar, double *param_ct_dev,
