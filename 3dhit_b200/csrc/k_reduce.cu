@@ -18,12 +18,11 @@ template <> __device__ __forceinline__ int shell_of<double>(double k2, double k0
   return (int)floor(__dadd_rn(__ddiv_rn(__dsqrt_rn(k2), k0), 0.5));
 }
 
-// Layout copies: a warp takes whole (x, y) rows, lanes along z, LC_UNROLL
+// Gather and box check: a warp takes whole (x, y) rows, lanes along z, LC_UNROLL
 // 32-mode chunks of the three components in flight per lane.  The row's
 // coordinates and offsets are formed once; with one mode per thread and a
 // division by each extent per mode, address arithmetic bound the box check
-// (256^3 float32: 52 us, now 31 = 0.68 of HBM; gather 29 -> 25; scatter 50 -> 53,
-// at the rate of its unaligned writes).
+// (256^3 float32: 52 us, now 31 = 0.68 of HBM; gather 29 -> 25).
 constexpr int LC_UNROLL = 2;
 constexpr int LC_WARPS = NT / 32;
 
@@ -89,31 +88,23 @@ template <typename T> cudaError_t launch_gather(const GatherArgs<T>& a, int nblo
 // ---------------------------------------------------------------------------
 // scatter: compact -> reference layout (modes outside the compact set are 0)
 // ---------------------------------------------------------------------------
+// A thread per mode over the whole grid: successive warps write one run of memory,
+// in whole lines.  With a warp per row (rows of Nz/2 + 1 entries start unaligned)
+// the writes took 10 to 14% longer: 512^3 float32 2/3 box 411 against 469 us, general
+// layout 565 against 634; 256^3 50 against 55; level at 128^3.
 template <typename T>
 __global__ void __launch_bounds__(NT) k_scatter(const V2<T>* __restrict__ cmp, V2<T>* __restrict__ ext, Geom g) {
-  const long long ce = (long long)g.Nx * g.Ny * g.Nzh, cc = (long long)g.Mx * g.My * g.Mzp;
-  const int lane = threadIdx.x & 31, nrows = g.Nx * g.Ny;
-  for (int row = blockIdx.x * LC_WARPS + (threadIdx.x >> 5); row < nrows; row += gridDim.x * LC_WARPS) {
-    const int fy = row % g.Ny, fx = row / g.Ny;
+  const long long nmodes = (long long)g.Nx * g.Ny * g.Nzh;
+  const long long cc = (long long)g.Mx * g.My * g.Mzp;
+  for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < nmodes; e += (long long)gridDim.x * NT) {
+    const int k = (int)(e % g.Nzh);
+    const long long r = e / g.Nzh;
+    const int fy = (int)(r % g.Ny), fx = (int)(r / g.Ny);
     const int i = compact_row(fx, g.hx, g.Mx, g.Nx), j = compact_row(fy, g.hy, g.My, g.Ny);
-    const int mz = i >= 0 && j >= 0 ? g.Mz : 0;  // stored modes of the row
-    const V2<T>* src = cmp + (mz ? ((long long)i * g.My + j) * g.Mzp : 0);
-    V2<T>* dst = ext + (long long)row * g.Nzh;
-    for (int k0 = lane; k0 < g.Nzh; k0 += 32 * LC_UNROLL) {
-      V2<T> v[LC_UNROLL][3];
+    const bool kept = i >= 0 && j >= 0 && k < g.Mz;
+    const long long m = kept ? ((long long)i * g.My + j) * g.Mzp + k : 0;
 #pragma unroll
-      for (int u = 0; u < LC_UNROLL; ++u) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) v[u][c] = k0 + 32 * u < mz ? src[c * cc + k0 + 32 * u] : czero<T>();
-      }
-#pragma unroll
-      for (int u = 0; u < LC_UNROLL; ++u) {
-        if (k0 + 32 * u < g.Nzh) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) dst[c * ce + k0 + 32 * u] = v[u][c];
-        }
-      }
-    }
+    for (int c = 0; c < 3; ++c) ext[c * nmodes + e] = kept ? cmp[c * cc + m] : czero<T>();
   }
 }
 
@@ -125,7 +116,7 @@ static int grid_for(long long n) {
 static int grid_rows(long long rows) { return grid_for(rows * 32); }
 
 template <typename T> cudaError_t launch_scatter(const V2<T>* cmp, V2<T>* ext, const Geom& g, cudaStream_t st) {
-  k_scatter<T><<<grid_rows((long long)g.Nx * g.Ny), NT, 0, st>>>(cmp, ext, g);
+  k_scatter<T><<<grid_for((long long)g.Nx * g.Ny * g.Nzh), NT, 0, st>>>(cmp, ext, g);
   return cudaGetLastError();
 }
 
