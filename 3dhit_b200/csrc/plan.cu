@@ -206,8 +206,7 @@ template <typename T> int ensure_path(hit_plan* p, int which) {
   if ((rc = ensure(P.D, cmp))) return rc;
   const int W = p3_tile_w<T>(g.Nx);
   P.p3_blocks = p3_num_blocks(g, W);
-  const long long nm = (long long)g.Mx * g.My * g.Mzp;
-  P.gather_blocks = (int)std::min<long long>((nm + NT - 1) / NT, 8 * 148);
+  P.gather_blocks = gather_grid(g);
   const int nb = std::max(P.p3_blocks, P.gather_blocks);
   if ((rc = ensure(P.partial, (size_t)3 * nb * sizeof(double)))) return rc;
   if ((rc = ensure(P.coef, COEF_BYTES))) return rc;
@@ -1347,7 +1346,7 @@ template <typename T> int gather_cotangent(hit_plan* p, const void* v, V2<T>* ds
   a.cmp = dst;
   a.g = make_geom(p->Nx, p->Ny, p->Nz, false);
   a.k = ktab_of<T>(p);
-  HIT_CK(launch_gather<T>(a, adj_blocks<T>(p), st));
+  HIT_CK(launch_gather<T>(a, gather_grid(a.g), st));
   return HIT_OK;
 }
 template <typename T> int scatter_cotangent(hit_plan* p, const V2<T>* v, void* dst, cudaStream_t st) {
