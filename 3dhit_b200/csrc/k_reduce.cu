@@ -18,69 +18,114 @@ template <> __device__ __forceinline__ int shell_of<double>(double k2, double k0
   return (int)floor(__dadd_rn(__ddiv_rn(__dsqrt_rn(k2), k0), 0.5));
 }
 
-// Gather and box check: a warp takes whole (x, y) rows, lanes along z, LC_UNROLL
-// 32-mode chunks of the three components in flight per lane.  The row's
-// coordinates and offsets are formed once; with one mode per thread and a
-// division by each extent per mode, address arithmetic bound the box check
-// (256^3 float32: 52 us, now 31 = 0.68 of HBM; gather 29 -> 25).
+// Layout copies and the box check take a mode per thread, or, where it is faster
+// (gather_by_rows, check_by_rows), whole (x, y) rows per warp, lanes along z,
+// LC_UNROLL 32-mode chunks of the three components in flight per lane.  The
+// row's coordinates and offsets are then formed once instead of with a division by
+// each extent per mode, whose arithmetic bounds large float32 grids; rows shorter
+// than a warp and grids with few rows leave lanes or warps idle.
 constexpr int LC_UNROLL = 2;
 constexpr int LC_WARPS = NT / 32;
 
 // ---------------------------------------------------------------------------
 // gather: reference layout -> compact layout (+ optional NSCAL partial sums)
 // ---------------------------------------------------------------------------
+template <typename T> struct GatherSums {  // a thread's share of the NSCAL sums
+  double E = 0, O = 0, B = 0;
+  __device__ __forceinline__ void add(const GatherArgs<T>& a, const V2<T> (&v)[3], T kx, T ky, int k) {
+    const T k2 = k2_of(kx, ky, a.k.kz[k]);
+    double a2 = 0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) a2 += (double)v[c].x * v[c].x + (double)v[c].y * v[c].y;
+    const double w = herm_weight(a.g, k);
+    E += w * a2;
+    O += w * (double)k2 * a2;
+    if (a.kmin2 <= k2 && k2 <= a.kmax2) B += w * a2;
+  }
+  __device__ __forceinline__ void store(const GatherArgs<T>& a, double* red) {
+    double r = block_sum_f64(E, red);
+    if (threadIdx.x == 0) a.partial[3 * blockIdx.x + 0] = r;
+    r = block_sum_f64(O, red);
+    if (threadIdx.x == 0) a.partial[3 * blockIdx.x + 1] = r;
+    r = block_sum_f64(B, red);
+    if (threadIdx.x == 0) a.partial[3 * blockIdx.x + 2] = r;
+  }
+};
+
 template <typename T>
 __global__ void __launch_bounds__(NT) k_gather(GatherArgs<T> a) {
+  __shared__ double red[32];
+  const Geom& g = a.g;
+  const long long nmodes = (long long)g.Mx * g.My * g.Mzp;
+  const long long ce = (long long)g.Nx * g.Ny * g.Nzh;  // ext comp stride
+  const long long cc = (long long)g.Mx * g.My * g.Mzp;  // compact comp stride
+  GatherSums<T> s;
+  for (long long m = blockIdx.x * (long long)NT + threadIdx.x; m < nmodes; m += (long long)gridDim.x * NT) {
+    const int k = (int)(m % g.Mzp);
+    const long long r = m / g.Mzp;
+    const int j = (int)(r % g.My), i = (int)(r / g.My);
+    V2<T> v[3] = {czero<T>(), czero<T>(), czero<T>()};
+    if (k < g.Mz) {
+      const int fx = full_pos(i, g.hx, g.Mx, g.Nx), fy = full_pos(j, g.hy, g.My, g.Ny);
+      const long long e = ((long long)fx * g.Ny + fy) * g.Nzh + k;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[c] = a.ext[c * ce + e];
+      if (a.partial) s.add(a, v, a.k.kx[fx], a.k.ky[fy], k);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) a.cmp[c * cc + m] = v[c];
+  }
+  if (a.partial) s.store(a, red);
+}
+
+__global__ void __launch_bounds__(NT) k_gather_rows(GatherArgs<float> a) {
   __shared__ double red[32];
   const Geom& g = a.g;
   const long long ce = (long long)g.Nx * g.Ny * g.Nzh;  // ext comp stride
   const long long cc = (long long)g.Mx * g.My * g.Mzp;  // compact comp stride
   const int lane = threadIdx.x & 31, nrows = g.Mx * g.My;
-  double sE = 0, sO = 0, sB = 0;
+  GatherSums<float> s;
   for (int row = blockIdx.x * LC_WARPS + (threadIdx.x >> 5); row < nrows; row += gridDim.x * LC_WARPS) {
     const int j = row % g.My, i = row / g.My;
     const int fx = full_pos(i, g.hx, g.Mx, g.Nx), fy = full_pos(j, g.hy, g.My, g.Ny);
-    const V2<T>* ext = a.ext + ((long long)fx * g.Ny + fy) * g.Nzh;
-    V2<T>* cmp = a.cmp + (long long)row * g.Mzp;
-    const T kx = a.k.kx[fx], ky = a.k.ky[fy];
+    const float2* ext = a.ext + ((long long)fx * g.Ny + fy) * g.Nzh;
+    float2* cmp = a.cmp + (long long)row * g.Mzp;
+    const float kx = a.k.kx[fx], ky = a.k.ky[fy];
     for (int k0 = lane; k0 < g.Mzp; k0 += 32 * LC_UNROLL) {
-      V2<T> v[LC_UNROLL][3];
+      float2 v[LC_UNROLL][3];
 #pragma unroll
       for (int u = 0; u < LC_UNROLL; ++u) {
         const int k = k0 + 32 * u;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) v[u][c] = k < g.Mz ? ext[c * ce + k] : czero<T>();
+        for (int c = 0; c < 3; ++c) v[u][c] = k < g.Mz ? ext[c * ce + k] : czero<float>();
       }
 #pragma unroll
       for (int u = 0; u < LC_UNROLL; ++u) {
         const int k = k0 + 32 * u;
         if (k >= g.Mzp) break;
-        if (a.partial && k < g.Mz) {
-          const T k2 = k2_of(kx, ky, a.k.kz[k]);
-          double a2 = 0;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) a2 += (double)v[u][c].x * v[u][c].x + (double)v[u][c].y * v[u][c].y;
-          const double w = herm_weight(g, k);
-          sE += w * a2;
-          sO += w * (double)k2 * a2;
-          if (a.kmin2 <= k2 && k2 <= a.kmax2) sB += w * a2;
-        }
+        if (a.partial && k < g.Mz) s.add(a, v[u], kx, ky, k);
 #pragma unroll
         for (int c = 0; c < 3; ++c) cmp[c * cc + k] = v[u][c];
       }
     }
   }
-  if (a.partial) {
-    double r = block_sum_f64(sE, red);
-    if (threadIdx.x == 0) a.partial[3 * blockIdx.x + 0] = r;
-    r = block_sum_f64(sO, red);
-    if (threadIdx.x == 0) a.partial[3 * blockIdx.x + 1] = r;
-    r = block_sum_f64(sB, red);
-    if (threadIdx.x == 0) a.partial[3 * blockIdx.x + 2] = r;
-  }
+  if (a.partial) s.store(a, red);
 }
 
+// float32 from 2^20 stored modes in rows of at least 128 points: 512^3 198 -> 171 us
+// (2/3 box), 256^3 29.6 -> 27.5 and 86 -> 71 (general layout), 128 x 128 x 512 16.0 ->
+// 14.8, general 128^3 14.0 -> 12.4; below, by rows: 128^3 6.5 -> 6.6, 64 x 64 x 1024 9.3 ->
+// 10.7, 512 x 512 x 8 11 -> 31, 256 x 256 x 64 10.8 -> 13.1; float64 256^3 44.9 -> 45.9.
+template <typename T> bool gather_by_rows(const Geom& g) {
+  return sizeof(T) == 4 && g.Nz >= 128 && (long long)g.Mx * g.My * g.Mzp >= (1 << 20);
+}
 template <typename T> cudaError_t launch_gather(const GatherArgs<T>& a, int nblocks, cudaStream_t st) {
+  if constexpr (sizeof(T) == 4) {
+    if (gather_by_rows<T>(a.g)) {
+      k_gather_rows<<<nblocks, NT, 0, st>>>(a);
+      return cudaGetLastError();
+    }
+  }
   k_gather<T><<<nblocks, NT, 0, st>>>(a);
   return cudaGetLastError();
 }

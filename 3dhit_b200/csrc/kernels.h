@@ -280,12 +280,11 @@ template <typename T> struct GatherArgs {
   double* partial;    // nullable: per-block NSCAL sums of the gathered state
 };
 
-// Blocks of a gather to the compact layout g (and rows of its partial): a warp per
-// row as far as one wave of eight blocks per SM goes.  Counted in modes, small grids
-// had two rows per warp one after another (32^3 3.7 us, 64^3 4.0).
+// Blocks of a gather to the compact layout g (and rows of its partial): a mode per
+// thread, at most one wave of eight blocks per SM.
 inline int gather_grid(const Geom& g) {
-  const int blocks = (g.Mx * g.My + NT / 32 - 1) / (NT / 32);
-  return blocks < 8 * 148 ? blocks : 8 * 148;
+  const long long blocks = ((long long)g.Mx * g.My * g.Mzp + NT - 1) / NT;
+  return (int)(blocks < 8 * 148 ? blocks : 8 * 148);
 }
 template <typename T> cudaError_t launch_gather(const GatherArgs<T>& a, int nblocks, cudaStream_t st);
 template <typename T> cudaError_t launch_scatter(const V2<T>* cmp, V2<T>* ext, const Geom& g, cudaStream_t st);
