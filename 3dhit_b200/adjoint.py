@@ -35,7 +35,23 @@ __all__ = ["rhs_vjp", "rk4_step_vjp", "rollout_vjp", "rollout_autograd", "PARAM_
 PARAM_NAMES = ("nu", "A", "eps")
 
 
-def _setup(rhs, params, u_hat, ct):
+# Modes from which one RHS transpose gains more on the 2/3 box than the box check
+# costs (a launch and a read back, 27 us).  On the general layout without it against
+# with it and the box: 64^3 float32 105 against 125 us, 4^3 75 against 105; 64 x 64 x 256
+# level (185; float64 315 against 282), 128^3 281 against 252.
+_BOX_CHECK_MODES = 1 << 19
+
+
+def _on_box(g, u_hat, steps):
+    """HIT_FLAG_ASSUME_DEALIASED where the transposes use it (fused columns: to
+    256 points along x, 128 in float64), pay for the check and u_hat is dealiased."""
+    fused = g.Nx <= (256 if g.dtype == torch.float32 else 128)
+    if not fused or (not steps and g.Nx * g.Ny * (g.Nz // 2 + 1) < _BOX_CHECK_MODES):
+        return 0
+    return resolve_flags(u_hat, g, None)
+
+
+def _setup(rhs, params, u_hat, ct, steps):
     if not isinstance(rhs, NSRHS):
         raise ValueError("the adjoint needs the package's own RHS (make_ns_rhs)")
     p = native_params(params.nu, params.forcing)
@@ -45,7 +61,7 @@ def _setup(rhs, params, u_hat, ct):
     u_hat = _check_state(u_hat, g)
     ct = _check_state(ct, g)
     # a dealiased state (one device check) lets the transposes carry the 2/3 box alone
-    p.flags |= resolve_flags(u_hat, g, None)
+    p.flags |= _on_box(g, u_hat, steps)
     return g, p, u_hat, ct
 
 
@@ -56,7 +72,7 @@ def _params_dict(pct):
 
 def rhs_vjp(rhs, u_hat, params, ct, t=0.0):
     """(d rhs / d u_hat)^T ct and the parameter cotangents."""
-    g, p, u_hat, ct = _setup(rhs, params, u_hat, ct)
+    g, p, u_hat, ct = _setup(rhs, params, u_hat, ct, 0)
     out = torch.empty_like(u_hat)
     pct = torch.zeros(3, dtype=torch.float64, device=u_hat.device)
     nat.call("hit_rhs_vjp", g.plan.handle, nat.ptr(u_hat), p, float(t), nat.ptr(ct), nat.ptr(out), nat.ptr(pct),
@@ -67,7 +83,7 @@ def rhs_vjp(rhs, u_hat, params, ct, t=0.0):
 def rk4_step_vjp(rhs, u_hat, params, dt, ct, t=0.0):
     """(d rk4_step / d u_hat)^T ct (stage inputs recomputed) and the parameter
     cotangents."""
-    g, p, u_hat, ct = _setup(rhs, params, u_hat, ct)
+    g, p, u_hat, ct = _setup(rhs, params, u_hat, ct, 1)
     out = torch.empty_like(u_hat)
     pct = torch.zeros(3, dtype=torch.float64, device=u_hat.device)
     nat.call("hit_rk4_step_vjp", g.plan.handle, nat.ptr(u_hat), p, float(dt), float(t), nat.ptr(ct), nat.ptr(out),
@@ -78,7 +94,7 @@ def rk4_step_vjp(rhs, u_hat, params, dt, ct, t=0.0):
 def rollout_vjp(rhs, u0, params, dt, nsteps, ct, t0=0.0, checkpoint_every=20):
     """(d rollout / d u0)^T ct with checkpoints every ``checkpoint_every``
     steps, and the parameter cotangents summed over the steps."""
-    g, p, u0, ct = _setup(rhs, params, u0, ct)
+    g, p, u0, ct = _setup(rhs, params, u0, ct, int(nsteps))
     out = torch.empty_like(u0)
     pct = torch.zeros(3, dtype=torch.float64, device=u0.device)
     nat.call("hit_rollout_vjp", g.plan.handle, nat.ptr(u0), p, float(dt), int(nsteps), float(t0),
