@@ -81,14 +81,23 @@ def kernel_alg_bytes(N, itemsize=8):
     Bx = N * M * Mz         # x-physical, (ky, kz) in the box
     Cx = N * N * Mz         # x,y-physical, kz in the box
     p3 = 3 * Bx + (51 * A + 18 * Bx) / 4.0  # mean over the 4 stages
+    plane = 8 <= N <= 64    # y-inverse, z pass and y-forward are one kernel (class z-pass)
     return {
         "x-inverse": (3 * A + 6 * Bx) * itemsize,
-        "y-inverse": (6 * Bx + 6 * Cx) * itemsize,
-        "z-pass": (6 * Cx + 3 * Cx) * itemsize,
-        "y-forward": (3 * Cx + 3 * Bx) * itemsize,
+        "y-inverse": 0.0 if plane else (6 * Bx + 6 * Cx) * itemsize,
+        "z-pass": (6 * Bx + 3 * Bx if plane else 6 * Cx + 3 * Cx) * itemsize,
+        "y-forward": 0.0 if plane else (3 * Cx + 3 * Bx) * itemsize,
         "x-forward+epilogue": p3 * itemsize,
         "forcing-coef": 0.0,
     }
+
+
+def launches_per_step(counts, steps):
+    """Kernels of one rollout step from the profiled launches per class: all but
+    the standalone x-inverse, which runs once per rollout (a stage is y-inverse,
+    z pass, y-forward, x-forward + epilogue and the forcing coefficient, the first
+    three in one kernel on small planes)."""
+    return sum(n for name, n in counts.items() if name != "x-inverse") // steps
 
 
 class ClockSampler:
@@ -754,7 +763,6 @@ def main():
         raise RuntimeError("non-finite energy after the timed rollout")
     ms_step = ms_max / args.steps
     value = job_rate(world, args.steps, ms_max)
-    launches_per_step = 4 * 5  # 4 x (y-inv, z, y-fwd, x-fwd+epi [+ next x-inverse], coef)
 
     # ---- per-kernel device times (events around every launch) -------------
     import ctypes
@@ -765,6 +773,7 @@ def main():
     prm = h3.forcing.native_params(NU, p.forcing, flags)
     nat.call("hit_profile_rollout", g.plan.handle, nat.ptr(u), prm, float(dt), args.profile_steps,
              nat.ptr(out), msa, cnt, nat.stream_ptr(dev))
+    per_step = launches_per_step(dict(zip(nat.KERNEL_CLASSES, cnt)), args.profile_steps)
     alg = kernel_alg_bytes(N) if not args.shape else {k: 0.0 for k in nat.KERNEL_CLASSES}
     per_kernel = {}
     for i, name in enumerate(nat.KERNEL_CLASSES):
@@ -843,7 +852,7 @@ def main():
                        "scheme": args.scheme},
             "grid_point_steps_per_s": value * N**3,
             "roofline": roofline, "step_roofline": step_model, "kernels": per_kernel,
-            "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches_per_step * args.steps + 1,
+            "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": per_step * args.steps + 1,
             "clocks": ck, "energy_end": E_end,
         }
         print(json.dumps(line), flush=True)

@@ -193,8 +193,9 @@ int hit_rollout_vjp(hit_plan *plan, const void *u0_hat,
  * HIT_NUM_KERNEL_CLASSES entries receive, per kernel class, the summed device
  * time in ms and the number of launches.  Classes: 0 x-inverse (P1),
  * 1 y-inverse, 2 z pass (c2r, u x w, r2c), 3 y-forward, 4 x-forward + RHS/RK4
- * epilogue (+ next stage's x-inverse), 5 forcing coefficient.  Synchronises
- * `stream` before returning. */
+ * epilogue (+ next stage's x-inverse), 5 forcing coefficient.  On the 2/3 box
+ * with Ny and Nz of 8 .. 64 classes 1 to 3 are one kernel, counted in class 2.
+ * Synchronises `stream` before returning. */
 #define HIT_NUM_KERNEL_CLASSES 6
 int hit_profile_rollout(hit_plan *plan, const void *u_hat,
                         const hit_params *params, double dt, int64_t nsteps,
