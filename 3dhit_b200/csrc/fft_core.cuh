@@ -406,10 +406,11 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
 }
-// The 64 bytes at gmem towards L2; no completion to wait for.  (As 64-byte bulk
-// prefetches, cp.async.bulk.prefetch.L2, the nine state rows per x position of an
-// RK4 stage cost more than they hid: x-forward pass 202 us against 168 at 256^3,
-// 17.2 against 11.0 at 64^3, 12.2 against 8.6 at 32^3.)
+// The start of a state row (64 bytes; 128 in float64 k_p3, one prefetch each) towards
+// L2; no completion to wait for.  (As 64-byte bulk prefetches,
+// cp.async.bulk.prefetch.L2, the nine state rows per x position of an RK4 stage cost
+// more than they hid: x-forward pass 202 us against 168 at 256^3, 17.2 against 11.0
+// at 64^3, 12.2 against 8.6 at 32^3.)
 __device__ __forceinline__ void prefetch_l2(const void* gmem) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(gmem));
 }

@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(NT) k_axis(AxisArgs<T> a, int nzt, int no, int
 template <typename T, int N> struct Axis2 {
   static constexpr int W = tile_w<T>(N);
   static constexpr int G = N * W / (N == 512 ? 32 : 16);
-    static constexpr int MINB = N == 512 ? 2 : (sizeof(T) == 8 ? 4 : 640 / G);
+  static constexpr int MINB = N == 512 ? 2 : (sizeof(T) == 8 ? 4 : 640 / G);
   using XT = XTile<N, W>;
   // exchange tile, twiddles, staged tile on a 128-byte boundary
   static constexpr size_t smem = sizeof(V2<T>) * (size_t)(XT::SLOTS + XT::TWS + N * W) + 128;
@@ -1034,10 +1034,13 @@ template <typename F> cudaError_t dispatch_len(int N, F&& f) {
   }
 }
 
-// lengths that k_axis serves (the column passes of shorter ones are k_col's)
-template <typename F> cudaError_t dispatch_long(int N, F&& f) {
+// lengths that k_axis serves (the column passes of shorter ones, and of 128
+// points in float64, are k_col's)
+template <typename T, typename F> cudaError_t dispatch_long(int N, F&& f) {
+  if constexpr (sizeof(T) == 4) {
+    if (N == 128) return f(std::integral_constant<int, 128>{});
+  }
   switch (N) {
-    case 128: return f(std::integral_constant<int, 128>{});
     case 256: return f(std::integral_constant<int, 256>{});
     case 512: return f(std::integral_constant<int, 512>{});
     case 1024: return f(std::integral_constant<int, 1024>{});
@@ -1114,7 +1117,7 @@ cudaError_t launch_axis(int N, bool inv, const AxisArgs<T>& a, int nzt, int no, 
   const long long ntiles = (long long)nzt * no * nc;
   if (col_pass<T>(N, inv, pf, ntiles * N * tile_w<T>(N) * (long long)sizeof(V2<T>)))
     return launch_col<T>(N, inv, a, nzt, no, nc, st);
-  return dispatch_long(N, [&](auto nn) {
+  return dispatch_long<T>(N, [&](auto nn) {
     constexpr int NN = decltype(nn)::value;
     constexpr int W = tile_w<T>(NN);
     if ((inv ? a.Mout : a.Min) != NN) return cudaErrorInvalidValue;  // the full side is all N rows
@@ -1327,8 +1330,8 @@ template <typename T> cudaError_t launch_p3(const P3Args<T>& a, cudaStream_t st)
 }
 
 template <typename T> cudaError_t prepare_axis_kernels(int Nx) {
-  if (Nx < 128) return cudaSuccess;
-  return dispatch_long(Nx, [&](auto nn) {
+  if (Nx < (sizeof(T) == 4 ? 128 : 256)) return cudaSuccess;
+  return dispatch_long<T>(Nx, [&](auto nn) {
     constexpr int NN = decltype(nn)::value;
     cudaError_t e;
     constexpr int W = tile_w<T>(NN);

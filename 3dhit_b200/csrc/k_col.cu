@@ -27,8 +27,8 @@ template <typename T, int N> struct ColCfg {
   static constexpr int GP = COL_THREADS / G;  // groups (tiles) per CTA
 };
 
-// ALL: every row of the compact side is stored (M = N).
-template <typename T, int N, bool INV, int ROWS>  // ROWS: 0 any, 1 the 2/3 box, 2 all rows
+// ROWS: the compact side stores 0 any rows, 1 the 2/3 box, 2 all of them (M = N)
+template <typename T, int N, bool INV, int ROWS>
 __global__ void __launch_bounds__(COL_THREADS, sizeof(T) == 4 ? 4 : 2) k_col(AxisArgs<T> a, int nzt, int no, int ntiles) {
   using C = ColCfg<T, N>;
   constexpr int W = C::W, G = C::G;

@@ -88,7 +88,7 @@ struct TrainSmem {
   uint32_t tslot;
 };
 
-// 32 columns [c0, c0 + 32) of row `row` of a K-major tile with 64 columns
+// columns [c, c + 8) of row `row` of a K-major tile with 64 columns
 __device__ __forceinline__ void store_bf16x8(unsigned char* tile, int row, int c, const float* v) {
   uint4 q;
   uint32_t* w = reinterpret_cast<uint32_t*>(&q);

@@ -6,8 +6,9 @@
 // What bounds small grids is the chain of dependent launches: at 32^3 each of
 // the three kernels took 4-5 us of mostly start-up, drain and L2 round trips.
 // Here the plane crosses shared memory in seven phases with a barrier between
-// them (RK4 step inside a rollout: 32^3 float32 67 -> 53 us, 64^3 107 -> 93,
-// 64^3 float64 160 -> 121; 512 x 32 x 32 334 -> 208; no shape served is slower).
+// them (RK4 step inside a rollout: 32^3 float32 67 -> 53 us, 64^3 107 -> 93, 64^3
+// float64 160 -> 121; 512 x 32 x 32 334 -> 208; no shape served is slower; plain
+// prefetches in the x passes later took the 32^3 step to 37).
 // The transforms are two-stage (N = R0 x R1) and in place: the inverse
 // ones decimate in frequency and leave their output permuted (index k at slot
 // (k mod R0) R1 + k / R0), u x w is formed value by value in that order, and

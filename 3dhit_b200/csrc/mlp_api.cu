@@ -15,7 +15,7 @@ int record_error(int code, const std::string& msg);
 namespace {
 using hit::MlpArgs;
 
-constexpr int MLP_GRID = 2 * 148;  // two 97 KB CTAs (256 TMEM columns each) per SM
+constexpr int MLP_GRID = 2 * 148;  // two 101 KB CTAs (256 TMEM columns each) per SM
 
 int cuda_err(cudaError_t e, const char* what) {
   return hit::record_error(HIT_E_CUDA, std::string(what) + ": " + cudaGetErrorString(e));

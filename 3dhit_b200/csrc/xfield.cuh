@@ -47,7 +47,8 @@ __device__ __forceinline__ void xf_twiddles(V2<T>* tws, const V2<T>* __restrict_
     tws[e] = tw[(e / X::R0 + 1) * (e % X::R0) * (TWN / N)];
 }
 
-// Stored rows of one side: compile-time when they are the 2/3 box (DA).
+// Stored rows of one side: compile-time when they are the 2/3 box (DA), so that the
+// bounds of a butterfly's positions fold into constants.
 template <int N, bool DA> struct ColRows {
   int h_, M_;
   __device__ __forceinline__ int h() const { return DA ? N / 3 + 1 : h_; }
@@ -63,22 +64,11 @@ template <int N, bool DA> struct ColRows {
   }
 };
 
-// The stored x rows: compile-time for the dealiased layout (DA), so that the
-// bounds of a butterfly's positions fold into constants.
-template <int N, bool DA> struct XRows {
-  int hx_, Mx_;
-  __device__ __forceinline__ explicit XRows(const Geom& g) : hx_(g.hx), Mx_(g.Mx) {}
-  __device__ __forceinline__ int hx() const { return DA ? N / 3 + 1 : hx_; }
-  __device__ __forceinline__ int Mx() const { return DA ? 2 * (N / 3) + 1 : Mx_; }
-  // stored row of position lo + b, b in [0, nb) (nb and lo constants), or -1
-  __device__ __forceinline__ int row(int b, int lo, int nb) const {
-    const int off = N - Mx();
-    if (DA && lo + nb <= hx()) return lo + b;
-    if (DA && lo >= hx() + off) return lo + b - off;
-    if (DA && lo >= hx() && lo + nb <= hx() + off) return -1;
-    const int pos = lo + b;
-    return pos < hx() ? pos : (pos >= hx() + off ? pos - off : -1);
-  }
+// The stored x rows.
+template <int N, bool DA> struct XRows : ColRows<N, DA> {
+  __device__ __forceinline__ explicit XRows(const Geom& g) : ColRows<N, DA>{g.hx, g.Mx} {}
+  __device__ __forceinline__ int hx() const { return this->h(); }
+  __device__ __forceinline__ int Mx() const { return this->M(); }
 };
 
 // Stage 0 of a group's transform in two parts: the loads of all its
